@@ -610,6 +610,7 @@ struct lu_batch_plan_t {
 namespace lub {
 int64_t batch_plan_size(const lu_batch_plan_t* p) { return p->batch; }
 const int32_t* batch_plan_dev_n(const lu_batch_plan_t* p) { return p->d_n; }
+const int32_t* batch_plan_dev_order(const lu_batch_plan_t* p) { return p->d_order; }
 int batch_plan_nmax(const lu_batch_plan_t* p) { return p->nmax; }
 }  // namespace lub
 

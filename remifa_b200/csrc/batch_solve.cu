@@ -1,15 +1,33 @@
 // Batched solves and adjoint for the factors a batch plan produced (new; the
 // reference has neither a batch nor a derivative).
 //
-// One warp per (matrix, right-hand side): the warp keeps b, x and the
-// residual of its column in shared memory (fp64) and works down the
-// triangles with the fp32 factors read straight from global memory:
-//   L x = b, U x = y   : column (axpy) form, column j of the factor read
-//                        coalesced by the 32 lanes;
-//   U^T z = g, L^T y = z: dot form, column j again, lane partial sums reduced
-//                        in a fixed shuffle tree (deterministic).
+// One CTA of eight warps per (matrix, group of up to NR right-hand sides); b,
+// x and the residual of the group live in shared memory (fp64), the fp32
+// factors and matrices are read from global memory / L2.
+//   * The 32 x 32 diagonal blocks of L and U are inverted once per item, in
+//     fp64, by substitution (one warp per block, lane j column j), and kept
+//     packed L^-1 \ U^-1 in shared memory; all 1 + refine_iters solves use
+//     them.
+//   * A triangle is then one step per block of 32 unknowns: x_t = Dinv_t (b_t -
+//     sum over the solved blocks), the sum split over the eight warps.  Not
+//     transposed: lanes are the block's rows, warp w sums the columns w, w +
+//     8, ...; transposed: warp w owns four of the block's columns, lanes run
+//     down the rows, one shuffle tree per column.  Both read the factor's
+//     columns coalesced.  While one warp multiplies by Dinv_t the others
+//     already sum block t+1's row over the blocks before t.
 // With the original fp32 matrices given, refine_iters rounds of FP64
-// refinement follow: r = b - op(A) x in fp64, x += op(LU)^-1 r.
+// refinement follow: r = b - op(A) x in fp64, x += op(LU)^-1 r.  Every sum has
+// a fixed order, so results do not depend on scheduling.
+//
+// What bounds it: the chain of dependent block steps (2 (1 + iters) n / 32 of
+// them, each an L2 latency and the inverse's product), hidden by three CTAs
+// per SM at n <= 256; there the factors of the resident matrices outgrow L2,
+// so every round reads them from DRAM again (2 TB/s).  The fp32 -> fp64
+// conversions (one warp instruction per 8 cycles and scheduler) take a
+// seventh of the time, the arithmetic less.  1,024 matrices of 64..256, one
+// right-hand side, 4 refinement rounds on B200: 0.44 ms (transposed 0.43),
+// 6.3 ms as one warp per (matrix, right-hand side) walking single columns.
+//
 // The adjoint of X = A^-1 B: dB = A^-T G (the transposed solve above, in
 // place in G) and dA = -dB X^T (fp64 dot products, stored fp32).
 #include "common.cuh"
@@ -24,108 +42,329 @@ namespace lub {
 // plan accessors (batch.cu)
 int64_t batch_plan_size(const lu_batch_plan_t* p);
 const int32_t* batch_plan_dev_n(const lu_batch_plan_t* p);
+const int32_t* batch_plan_dev_order(const lu_batch_plan_t* p);
 int batch_plan_nmax(const lu_batch_plan_t* p);
 
 namespace {
 
-constexpr int kWarpsPerCta = 4;
+constexpr int kWarps = 8;
+constexpr int kT = 32 * kWarps;
+constexpr int BS = 32;                 // unknowns per step
+constexpr int kDS = BS + 1;            // row stride of an inverted block (doubles)
 
-// x (shared, fp64, length n) <- L^-1 x, L unit lower (fp32, column-major).
-__device__ __forceinline__ void lower_solve(const float* __restrict__ F, int64_t ld,
-                                            int n, double* x) {
-  const int lane = threadIdx.x & 31;
-  for (int j = 0; j < n - 1; ++j) {
-    __syncwarp();
-    const double xj = x[j];
-    const float* col = F + (int64_t)j * ld;
-    for (int i = j + 1 + lane; i < n; i += 32) x[i] = fma(-(double)col[i], xj, x[i]);
-  }
-  __syncwarp();
+// Shared memory of one item, in doubles: inverted diagonal blocks, x, b and r of
+// the group, the warps' partial sums.
+__host__ __device__ inline size_t smem_doubles(int nmax, int nr) {
+  const size_t nb = (size_t)(nmax + BS - 1) / BS;
+  return nb * BS * kDS + 3 * nb * BS * nr + (size_t)kWarps * nr * BS;
 }
 
-// x <- U^-1 x, U upper with its diagonal (column form, bottom up).
-__device__ __forceinline__ void upper_solve(const float* __restrict__ F, int64_t ld,
-                                            int n, double* x) {
-  const int lane = threadIdx.x & 31;
-  for (int j = n - 1; j >= 0; --j) {
+// Inverses of the unit lower and the upper triangle of every diagonal block,
+// packed in place of the block at S + t BS kDS (row-major, stride kDS), one
+// warp per block.  The 16 x 16 diagonal halves by substitution (half-warp h
+// half h, lane j column j), then the off-diagonal quarters as products:
+// -L22^-1 L21 L11^-1 by the lower half-warp, -U11^-1 U12 U22^-1 by the upper
+// one (half the registers of a 32-row substitution, so three CTAs fit; a
+// rolled form of this code took 25 us more on 1,024 matrices of 64..256).
+__device__ __forceinline__ void invert_blocks(const float* __restrict__ F, int64_t ld, int n,
+                                              int nb, double* S) {
+  constexpr int H = BS / 2;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int h = lane >> 4, j = lane & (H - 1);
+#pragma unroll 1
+  for (int t = warp; t < nb; t += kWarps) {
+    double* D = S + (size_t)t * BS * kDS;
+    const int r0 = t * BS;
+    const bool rowok = r0 + lane < n;
+    const float* src = F + (r0 + lane) + (int64_t)r0 * ld;
+#pragma unroll 16
+    for (int c = 0; c < BS; ++c) {
+      const bool ok = rowok && r0 + c < n;
+      D[lane * kDS + c] = ok ? (double)src[(int64_t)c * ld] : (c == lane ? 1.0 : 0.0);
+    }
     __syncwarp();
-    const float* col = F + (int64_t)j * ld;
-    const double xj = x[j] / (double)col[j];
-    __syncwarp();
-    if (lane == 0) x[j] = xj;
-    for (int i = lane; i < j; i += 32) x[i] = fma(-(double)col[i], xj, x[i]);
-  }
-  __syncwarp();
-}
-
-__device__ __forceinline__ double warp_sum(double v) {
+    double* Dh = D + h * H * (kDS + 1);
+    const double rd = 1.0 / D[lane * kDS + lane];
+    {
+      double z[H];
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      for (int i = 0; i < H; ++i) z[i] = i == j ? 1.0 : 0.0;
+#pragma unroll
+      for (int k = 0; k < H; ++k)
+#pragma unroll
+        for (int i = k + 1; i < H; ++i) z[i] = fma(-Dh[i * kDS + k], z[k], z[i]);
+      __syncwarp();  // every read of L is done
+#pragma unroll
+      for (int i = 1; i < H; ++i)
+        if (i > j) Dh[i * kDS + j] = z[i];
+#pragma unroll
+      for (int i = 0; i < H; ++i) z[i] = i == j ? rd : 0.0;
+#pragma unroll
+      for (int k = H - 1; k >= 0; --k) {
+        // row k takes its reciprocal in the columns right of k; the columns
+        // left of k have nothing there
+        const double rk = __shfl_sync(0xffffffffu, rd, h * H + k);
+        if (k < j) z[k] *= rk;
+#pragma unroll
+        for (int i = 0; i < k; ++i) z[i] = fma(-Dh[i * kDS + k], z[k], z[i]);
+      }
+      __syncwarp();  // every read of U is done
+#pragma unroll
+      for (int i = 0; i < H; ++i)
+        if (i <= j) Dh[i * kDS + j] = z[i];
+    }
+    __syncwarp();
+    double* P = h ? D + H : D + H * kDS;              // U12 or L21
+    const double* Q = h ? D : D + H * (kDS + 1);      // U11^-1 or L22^-1
+    double a[H], w[H];
+#pragma unroll
+    for (int k = 0; k < H; ++k)
+      a[k] = (h ? k <= j : k > j) ? Dh[k * kDS + j] : (k == j ? 1.0 : 0.0);
+#pragma unroll
+    for (int i = 0; i < H; ++i) {
+      w[i] = 0.0;
+#pragma unroll
+      for (int k = 0; k < H; ++k) w[i] = fma(P[i * kDS + k], a[k], w[i]);
+    }
+    __syncwarp();  // every read of the quarters is done
+#pragma unroll
+    for (int i = 0; i < H; ++i) {
+      double v = h ? Q[i * kDS + i] * w[i] : w[i];
+#pragma unroll
+      for (int k = 0; k < H; ++k)
+        if (h ? k > i : k < i) v = fma(Q[i * kDS + k], w[k], v);
+      P[i * kDS + j] = -v;
+    }
+  }
+}
+
+// Row lane of the packed inverse (transposed: column lane) times y (16-byte
+// aligned).  lower: L^-1 (unit diagonal) else U^-1.  Entries of the other
+// triangle are skipped.
+__device__ __forceinline__ double dinv_mul(const double* D, bool trans, bool lower,
+                                           const double* y) {
+  const int lane = threadIdx.x & 31;
+  const bool below = lower != trans;  // op(triangle) is lower
+  const double own = lower ? 1.0 : D[lane * kDS + lane];
+  const double* d = trans ? D + lane : D + lane * kDS;
+  const int st = trans ? kDS : 1;
+  double s[4] = {own * y[lane], 0.0, 0.0, 0.0};
+#pragma unroll
+  for (int k = 0; k < BS; k += 2) {
+    const double2 y2 = *reinterpret_cast<const double2*>(y + k);
+    if (below ? k < lane : k > lane) s[k & 3] = fma(d[k * st], y2.x, s[k & 3]);
+    if (below ? k + 1 < lane : k + 1 > lane)
+      s[(k + 1) & 3] = fma(d[(k + 1) * st], y2.y, s[(k + 1) & 3]);
+  }
+  return (s[0] + s[1]) + (s[2] + s[3]);
+}
+
+// Sums of four per-lane partials over the 32 lanes: two halving exchanges,
+// then three full steps.  Lanes 8 q .. 8 q + 7 end with sum q.
+__device__ __forceinline__ double reduce4(const double (&a)[4]) {
+  const int lane = threadIdx.x & 31;
+  const bool b4 = lane & 16, b3 = lane & 8;
+  double v0 = (b4 ? a[2] : a[0]) + __shfl_xor_sync(0xffffffffu, b4 ? a[0] : a[2], 16);
+  double v1 = (b4 ? a[3] : a[1]) + __shfl_xor_sync(0xffffffffu, b4 ? a[1] : a[3], 16);
+  double v = (b3 ? v1 : v0) + __shfl_xor_sync(0xffffffffu, b3 ? v0 : v1, 8);
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
 
-// x <- U^-T x (dot form, top down: x_j = (x_j - U[0:j, j] . x[0:j]) / U_jj).
-__device__ __forceinline__ void upper_t_solve(const float* __restrict__ F, int64_t ld,
-                                              int n, double* x) {
-  const int lane = threadIdx.x & 31;
-  for (int j = 0; j < n; ++j) {
-    const float* col = F + (int64_t)j * ld;
-    double p = 0.0;
-    for (int i = lane; i < j; i += 32) p = fma((double)col[i], x[i], p);
-    p = warp_sum(p);
-    if (lane == 0) x[j] = (x[j] - p) / (double)col[j];
-    __syncwarp();
-  }
-}
+// The warp's share of rows [r0, r0 + 32) of op(F) times x over whole blocks of
+// 32 columns: not transposed, lane = row, columns 4 warp .. 4 warp + 3 of each
+// block; transposed, rows 4 warp .. 4 warp + 3 of the row block (columns of
+// F), lanes over the block's 32.  Rows and columns past n read the last valid
+// one instead: x is zero there, and sums of rows past n are dropped.
+template <bool TRANS, int NR>
+struct Partial {
+  static constexpr int NA = TRANS ? 4 : 1;
+  double acc[NA][NR];
+  const float* p[4];  // column 4 warp + q of F (transposed: r0 + 4 warp + q, from row lane)
+  int row;            // lane's row (not transposed)
 
-// x <- L^-T x (dot form, bottom up: x_j = x_j - L[j+1:n, j] . x[j+1:n]).
-__device__ __forceinline__ void lower_t_solve(const float* __restrict__ F, int64_t ld,
-                                              int n, double* x) {
-  const int lane = threadIdx.x & 31;
-  for (int j = n - 2; j >= 0; --j) {
-    const float* col = F + (int64_t)j * ld;
-    double p = 0.0;
-    for (int i = j + 1 + lane; i < n; i += 32) p = fma((double)col[i], x[i], p);
-    p = warp_sum(p);
-    if (lane == 0) x[j] = x[j] - p;
-    __syncwarp();
+  __device__ __forceinline__ void init(const float* __restrict__ F, int64_t ld) {
+    const int warp = threadIdx.x >> 5;
+    if (!TRANS) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) p[q] = F + (4 * warp + q) * ld;
+    }
   }
-}
-
-__device__ __forceinline__ void solve(const float* F, int64_t ld, int n, double* x,
-                                      bool trans) {
-  if (!trans) {
-    lower_solve(F, ld, n, x);
-    upper_solve(F, ld, n, x);
-  } else {
-    upper_t_solve(F, ld, n, x);
-    lower_t_solve(F, ld, n, x);
+  // the row block of the next sums
+  __device__ __forceinline__ void start(const float* __restrict__ F, int64_t ld, int n, int r0) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (!TRANS) {
+      row = min(r0 + lane, n - 1);
+    } else {
+      const float* c = F + lane + (r0 + 4 * warp) * ld;
+      if (r0 + BS <= n) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) p[q] = c + q * ld;
+      } else {
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          p[q] = F + lane + (int64_t)min(r0 + 4 * warp + q, n - 1) * ld;
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < NA; ++q)
+#pragma unroll
+      for (int c = 0; c < NR; ++c) acc[q][c] = 0.0;
   }
-}
+  // The warp's entries of block q0: of a whole block, of any (the last valid
+  // row / column in place of those past n).
+  __device__ __forceinline__ void fetch_whole(float (&v)[4], int64_t ld, int q0) const {
+    const int64_t at = TRANS ? (int64_t)(q0 * BS) : row + q0 * (BS * ld);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) v[q] = p[q][at];
+  }
+  __device__ __forceinline__ void fetch(float (&v)[4], int64_t ld, int n, int q0) const {
+    if ((q0 + 1) * BS <= n) return fetch_whole(v, ld, q0);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t at = TRANS ? (int64_t)(q0 * BS) : row + q0 * (BS * ld);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int over = max(0, q0 * BS + (TRANS ? lane : 4 * warp + q) - (n - 1));
+      v[q] = p[q][at - over * (TRANS ? 1 : ld)];
+    }
+  }
+  // block q0's entries v times x
+  __device__ __forceinline__ void add(const float (&v)[4], int q0, const double* x, int np) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int c = 0; c < NR; ++c) {
+      const double* xc = x + c * np + q0 * BS;
+      if (TRANS) {
+        const double xv = xc[lane];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) acc[q][c] = fma((double)v[q], xv, acc[q][c]);
+      } else {
+        const double2 x0 = *reinterpret_cast<const double2*>(xc + 4 * warp);
+        const double2 x1 = *reinterpret_cast<const double2*>(xc + 4 * warp + 2);
+        acc[0][c] = fma((double)v[0], x0.x, acc[0][c]);
+        acc[0][c] = fma((double)v[1], x0.y, acc[0][c]);
+        acc[0][c] = fma((double)v[2], x1.x, acc[0][c]);
+        acc[0][c] = fma((double)v[3], x1.y, acc[0][c]);
+      }
+    }
+  }
+  // M whole blocks from q0, their loads all in flight before the first use
+  template <int M>
+  __device__ __forceinline__ void add_whole(int64_t ld, int q0, const double* x, int np) {
+    float v[M][4];
+#pragma unroll
+    for (int u = 0; u < M; ++u) fetch_whole(v[u], ld, q0 + u);
+#pragma unroll
+    for (int u = 0; u < M; ++u) add(v[u], q0 + u, x, np);
+  }
+  // blocks q0 .. q1 - 1
+  __device__ __forceinline__ void add_range(int64_t ld, int n, int q0, int q1, const double* x,
+                                            int np) {
+    const int full = min(q1, n / BS);
+    float vt[4];
+    if (full < q1) fetch(vt, ld, n, full);
+#pragma unroll 1
+    for (; q0 + 4 <= full; q0 += 4) add_whole<4>(ld, q0, x, np);
+    if (full - q0 == 3) add_whole<3>(ld, q0, x, np);
+    else if (full - q0 == 2) add_whole<2>(ld, q0, x, np);
+    else if (full - q0 == 1) add_whole<1>(ld, q0, x, np);
+    if (full < q1) add(vt, full, x, np);
+  }
 
-// r = b - op(A) x (A fp32, fp64 arithmetic).
-__device__ __forceinline__ void residual(const float* __restrict__ A, int64_t ld, int n,
-                                         const double* b, const double* x, double* r,
-                                         bool trans) {
-  const int lane = threadIdx.x & 31;
-  if (!trans) {
-    for (int i = lane; i < n; i += 32) r[i] = b[i];
-    for (int j = 0; j < n; ++j) {
+  // Partial sums to part: [warp][c][row] not transposed, [c][row] transposed
+  __device__ __forceinline__ void publish(double* part) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int c = 0; c < NR; ++c) {
+      if (!TRANS) {
+        part[(warp * NR + c) * BS + lane] = acc[0][c];
+      } else {
+        const double a[4] = {acc[0][c], acc[NA > 1 ? 1 : 0][c], acc[NA > 2 ? 2 : 0][c],
+                             acc[NA > 3 ? 3 : 0][c]};
+        const double v = reduce4(a);
+        if ((lane & 7) == 0) part[c * BS + 4 * warp + (lane >> 3)] = v;
+      }
+    }
+  }
+  // Sum of row lane of column c (after a CTA barrier)
+  static __device__ __forceinline__ double total(const double* part, int c) {
+    const int lane = threadIdx.x & 31;
+    if (TRANS) return part[c * BS + lane];
+    double s = part[c * BS + lane];
+#pragma unroll
+    for (int w = 1; w < kWarps; ++w) s += part[(w * NR + c) * BS + lane];
+    return s;
+  }
+};
+
+// x <- op(T)^-1 x for the lower (unit) or upper triangle of F; all threads.
+// Ends with a CTA barrier.
+template <bool TRANS, int NR>
+__device__ __forceinline__ void tri_solve(const float* __restrict__ F, int64_t ld, int n, int nb,
+                                          bool lower, const double* S, double* x, int np,
+                                          double* part) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const bool fwd = lower != TRANS;
+  Partial<TRANS, NR> p;
+  float pv[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+  p.init(F, ld);
+  p.start(F, ld, n, (fwd ? 0 : nb - 1) * BS);
+#pragma unroll 1
+  for (int s = 0; s < nb; ++s) {
+    const int t = fwd ? s : nb - 1 - s;
+    if (s > 0) p.add(pv, fwd ? t - 1 : t + 1, x, np);
+    p.publish(part);
+    __syncthreads();
+    if (s + 1 < nb) {
+      p.start(F, ld, n, (fwd ? t + 1 : t - 1) * BS);
+      p.fetch(pv, ld, n, t);
+    }
+    if (warp < NR) {
+      double* xc = x + warp * np + t * BS;
+      // rows past n stay zero whatever the sums hold
+      const bool ok = t * BS + lane < n;
+      const double y = xc[lane] - Partial<TRANS, NR>::total(part, warp);
+      xc[lane] = ok ? y : 0.0;
       __syncwarp();
-      const double xj = x[j];
-      const float* col = A + (int64_t)j * ld;
-      for (int i = lane; i < n; i += 32) r[i] = fma(-(double)col[i], xj, r[i]);
+      const double v = dinv_mul(S + (size_t)t * BS * kDS, TRANS, lower, xc);
+      __syncwarp();
+      xc[lane] = ok ? v : 0.0;
     }
-  } else {
-    for (int j = 0; j < n; ++j) {
-      const float* col = A + (int64_t)j * ld;
-      double p = 0.0;
-      for (int i = lane; i < n; i += 32) p = fma((double)col[i], x[i], p);
-      p = warp_sum(p);
-      if (lane == 0) r[j] = b[j] - p;
+    // the blocks solved before t
+    if (s > 0 && s + 1 < nb) p.add_range(ld, n, fwd ? 0 : t + 1, fwd ? t : nb, x, np);
+    __syncthreads();
+  }
+}
+
+template <bool TRANS, int NR>
+__device__ __forceinline__ void solve(const float* F, int64_t ld, int n, int nb, const double* S,
+                                      double* x, int np, double* part) {
+  tri_solve<TRANS, NR>(F, ld, n, nb, !TRANS, S, x, np, part);
+  tri_solve<TRANS, NR>(F, ld, n, nb, TRANS, S, x, np, part);
+}
+
+// r = b - op(A) x (A fp32, fp64 arithmetic), one row block per barrier pair.
+template <bool TRANS, int NR>
+__device__ __forceinline__ void residual(const float* __restrict__ A, int64_t ld, int n, int nb,
+                                         const double* b, const double* x, double* r, int np,
+                                         double* part) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  Partial<TRANS, NR> p;
+  p.init(A, ld);
+#pragma unroll 1
+  for (int t = 0; t < nb; ++t) {
+    p.start(A, ld, n, t * BS);
+    p.add_range(ld, n, 0, nb, x, np);
+    __syncthreads();  // the previous block's sums are read
+    p.publish(part);
+    __syncthreads();
+    if (warp < NR) {
+      const int i = warp * np + t * BS + lane;
+      r[i] = t * BS + lane < n ? b[i] - Partial<TRANS, NR>::total(part, warp) : 0.0;
     }
   }
-  __syncwarp();
+  __syncthreads();
 }
 
 struct SolveArgs {
@@ -137,78 +376,104 @@ struct SolveArgs {
   const int32_t* n;
   int64_t batch;
   int nrhs;
-  int trans;
   int iters;
-  int nmax;
+  const int32_t* order;     // matrices by decreasing size
 };
 
-__global__ void __launch_bounds__(32 * kWarpsPerCta)
+template <bool TRANS, int NR>
+__global__ void __launch_bounds__(kT, 3)
 batch_solve_kernel(SolveArgs s) {
-  extern __shared__ double sh[];
-  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  double* xb = sh + (size_t)wid * 3 * s.nmax;
-  double* bb = xb + s.nmax;
-  double* rb = bb + s.nmax;
-  const int64_t items = s.batch * s.nrhs;
-  for (int64_t it = (int64_t)blockIdx.x * kWarpsPerCta + wid; it < items;
-       it += (int64_t)gridDim.x * kWarpsPerCta) {
-    const int64_t m = it / s.nrhs;
-    const int c = (int)(it - m * s.nrhs);
-    const int n = s.n[m];
-    const float* F = s.lu[m];
-    const int64_t ldf = s.ldlu ? s.ldlu[m] : n;
-    double* xg = s.x[m] + (int64_t)c * n;
-    for (int i = lane; i < n; i += 32) {
-      xb[i] = xg[i];
-      bb[i] = xg[i];
+  extern __shared__ __align__(16) double sh[];
+  const int groups = (s.nrhs + NR - 1) / NR;
+  const int64_t item = blockIdx.x;
+  const int64_t m = s.order[item / groups];
+  const int c0 = (int)(item % groups) * NR;
+  const int nc = min(NR, s.nrhs - c0);
+  const int n = s.n[m];
+  const int nb = (n + BS - 1) / BS, np = nb * BS;
+  double* S = sh;
+  double* xb = S + (size_t)nb * BS * kDS;
+  double* bb = xb + (size_t)NR * np;
+  double* rb = bb + (size_t)NR * np;
+  double* part = rb + (size_t)NR * np;
+  const float* F = s.lu[m];
+  const int64_t ldf = s.ldlu ? s.ldlu[m] : n;
+  double* xg = s.x[m] + (int64_t)c0 * n;
+  for (int e = threadIdx.x; e < NR * np; e += kT) {
+    const int c = e / np, i = e - c * np;
+    const double v = (c < nc && i < n) ? xg[i + (int64_t)c * n] : 0.0;
+    xb[e] = v;
+    bb[e] = v;
+  }
+  invert_blocks(F, ldf, n, nb, S);
+  __syncthreads();
+  solve<TRANS, NR>(F, ldf, n, nb, S, xb, np, part);
+  if (s.a) {
+    const float* A = s.a[m];
+    const int64_t lda = s.lda ? s.lda[m] : n;
+    for (int k = 0; k < s.iters; ++k) {
+      residual<TRANS, NR>(A, lda, n, nb, bb, xb, rb, np, part);
+      solve<TRANS, NR>(F, ldf, n, nb, S, rb, np, part);
+      for (int e = threadIdx.x; e < NR * np; e += kT) xb[e] += rb[e];
+      __syncthreads();
     }
-    __syncwarp();
-    solve(F, ldf, n, xb, s.trans != 0);
-    if (s.a) {
-      const float* A = s.a[m];
-      const int64_t lda = s.lda ? s.lda[m] : n;
-      for (int k = 0; k < s.iters; ++k) {
-        residual(A, lda, n, bb, xb, rb, s.trans != 0);
-        solve(F, ldf, n, rb, s.trans != 0);
-        for (int i = lane; i < n; i += 32) xb[i] += rb[i];
-        __syncwarp();
-      }
-    }
-    for (int i = lane; i < n; i += 32) xg[i] = xb[i];
-    __syncwarp();
+  }
+  for (int e = threadIdx.x; e < nc * np; e += kT) {
+    const int c = e / np, i = e - c * np;
+    if (i < n) xg[i + (int64_t)c * n] = xb[e];
   }
 }
 
-// dA_m[i, j] = -sum_r dB_m[i, r] X_m[j, r], one CTA per matrix.
-__global__ void __launch_bounds__(256)
+// dA_m[i, j] = -sum_r dB_m[i, r] X_m[j, r], one CTA per matrix (largest
+// first): warps take columns j, lanes rows i, dB and X through L1; the writes
+// of dA bound it (1,024 matrices of 64..256: 38 us = 3.0 TB/s; 147 us with an
+// index division per element).
+__global__ void __launch_bounds__(kT)
 batch_outer_kernel(const double* const* __restrict__ db, const double* const* __restrict__ x,
                    float* const* __restrict__ da, const int32_t* __restrict__ ldda,
-                   const int32_t* __restrict__ ns, int nrhs) {
-  const int m = blockIdx.x;
+                   const int32_t* __restrict__ ns, const int32_t* __restrict__ order, int nrhs) {
+  const int m = order[blockIdx.x];
   const int n = ns[m];
   const int64_t ld = ldda ? (int64_t)ldda[m] : n;
-  const double* G = db[m];
-  const double* X = x[m];
-  float* D = da[m];
-  for (int64_t e = threadIdx.x; e < (int64_t)n * n; e += blockDim.x) {
-    const int j = (int)(e / n), i = (int)(e - (int64_t)j * n);
-    double acc = 0.0;
-    for (int r = 0; r < nrhs; ++r)
-      acc = fma(G[i + (int64_t)r * n], X[j + (int64_t)r * n], acc);
-    D[i + j * ld] = (float)(-acc);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const double* __restrict__ G = db[m];
+  const double* __restrict__ X = x[m];
+  float* __restrict__ D = da[m];
+  constexpr int CW = 4;  // columns of a warp per pass over the rows
+  for (int j0 = CW * warp; j0 < n; j0 += CW * kWarps) {
+    for (int i = lane; i < n; i += 32) {
+      double acc[CW] = {0.0, 0.0, 0.0, 0.0};
+      for (int r = 0; r < nrhs; ++r) {
+        const double g = G[i + (int64_t)r * n];
+#pragma unroll
+        for (int q = 0; q < CW; ++q)
+          if (j0 + q < n) acc[q] = fma(g, X[j0 + q + (int64_t)r * n], acc[q]);
+      }
+#pragma unroll
+      for (int q = 0; q < CW; ++q)
+        if (j0 + q < n) D[i + (j0 + q) * ld] = (float)(-acc[q]);
+    }
   }
 }
 
-lu_status launch_batch_solve(cudaStream_t st, const SolveArgs& s) {
-  if (s.batch == 0 || s.nrhs == 0) return LU_SUCCESS;
-  const size_t smem = (size_t)kWarpsPerCta * 3 * s.nmax * sizeof(double);
-  LUB_CUDA_TRY(set_smem_limit((const void*)batch_solve_kernel, smem));
-  const int64_t items = s.batch * s.nrhs;
-  const int64_t grid = std::min<int64_t>((items + kWarpsPerCta - 1) / kWarpsPerCta,
-                                         (int64_t)sm_count() * 16);
-  batch_solve_kernel<<<(unsigned)grid, 32 * kWarpsPerCta, smem, st>>>(s);
+template <bool TRANS, int NR>
+lu_status launch_solve(cudaStream_t st, const SolveArgs& s, int nmax) {
+  const size_t smem = smem_doubles(nmax, NR) * sizeof(double);
+  const int64_t items = s.batch * ((s.nrhs + NR - 1) / NR);
+  if (items > 0x7fffffffll) return LU_ERR_INVALID_ARG;
+  LUB_CUDA_TRY(set_smem_limit((const void*)batch_solve_kernel<TRANS, NR>, smem));
+  batch_solve_kernel<TRANS, NR><<<(unsigned)items, kT, smem, st>>>(s);
   LUB_LAUNCH_CHECK();
   return LU_SUCCESS;
+}
+
+// Right-hand sides per CTA: a second and a fourth column reuse the factor
+// entries already loaded and the inverted blocks.
+template <bool TRANS>
+lu_status launch_batch_solve(cudaStream_t st, const SolveArgs& s, int nmax) {
+  if (s.nrhs == 1) return launch_solve<TRANS, 1>(st, s, nmax);
+  if (s.nrhs == 2) return launch_solve<TRANS, 2>(st, s, nmax);
+  return launch_solve<TRANS, 4>(st, s, nmax);
 }
 
 }  // namespace
@@ -237,10 +502,11 @@ LU_API lu_status lu_batch_solve_c(lu_batch_plan plan, lu_stream_t stream,
   s.n = batch_plan_dev_n(plan);
   s.batch = batch;
   s.nrhs = nrhs;
-  s.trans = trans;
   s.iters = d_a ? refine_iters : 0;
-  s.nmax = batch_plan_nmax(plan);
-  return launch_batch_solve((cudaStream_t)stream, s);
+  s.order = batch_plan_dev_order(plan);
+  const int nmax = batch_plan_nmax(plan);
+  return trans ? launch_batch_solve<true>((cudaStream_t)stream, s, nmax)
+               : launch_batch_solve<false>((cudaStream_t)stream, s, nmax);
 }
 
 LU_API lu_status lu_batch_adjoint_c(lu_batch_plan plan, lu_stream_t stream,
@@ -257,8 +523,9 @@ LU_API lu_status lu_batch_adjoint_c(lu_batch_plan plan, lu_stream_t stream,
   LUB_TRY(lu_batch_solve_c(plan, stream, d_lu, d_ldlu, d_a, d_lda, d_g, nrhs, 1,
                            refine_iters));
   if (d_da) {
-    batch_outer_kernel<<<(unsigned)batch, 256, 0, st>>>(d_g, d_x, d_da, d_ldda,
-                                                        batch_plan_dev_n(plan), nrhs);
+    batch_outer_kernel<<<(unsigned)batch, kT, 0, st>>>(d_g, d_x, d_da, d_ldda,
+                                                       batch_plan_dev_n(plan),
+                                                       batch_plan_dev_order(plan), nrhs);
     LUB_LAUNCH_CHECK();
   }
   return LU_SUCCESS;
