@@ -6,7 +6,6 @@
 namespace lub {
 
 // panel.cu
-size_t diag_smem_bytes(int w);
 lu_status launch_diag_factor(cudaStream_t st, float* a, int64_t lda, int w,
                              int64_t col0, int* first_bad);
 // Low-precision K-major copies a panel launch also writes (fp16 or bf16:
