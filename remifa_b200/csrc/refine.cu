@@ -144,7 +144,7 @@ lu_status refine_multi(lu_stream_t stream, int64_t n, int64_t nrhs, const float*
     if (std::isnan(e) || e <= tol || it >= max_iter) break;
     LUB_CUDA_TRY(cudaMemcpyAsync(D, R, (size_t)n * nrhs * 8, cudaMemcpyDeviceToDevice, st));
     LUB_TRY(launch_lu_solve(st, n, d_lu, ldlu, D, n, nrhs, trans != 0, sync, R));
-    for (int64_t c = 0; c < nrhs; ++c) LUB_TRY(launch_axpy(st, n, D + c * n, d_x + c * ldx));
+    LUB_TRY(launch_axpy(st, n, nrhs, D, d_x, ldx));
     ++it;
   }
   if (iters) *iters = it;

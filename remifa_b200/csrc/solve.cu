@@ -27,6 +27,7 @@
 // lane and one shuffle reduction after x_{t-1} lands.
 #include "common.cuh"
 #include "kernels.cuh"
+#include "mma64.cuh"
 #include "solve.cuh"
 
 namespace lub {
@@ -934,146 +935,216 @@ rowsum_final_kernel(int64_t n, int nchunks, const double* __restrict__ P,
   if ((threadIdx.x & 31) == 0) atomicMax(out, (unsigned long long)__double_as_longlong(s));
 }
 
-__global__ void axpy_kernel(int64_t n, const double* __restrict__ d,
-                            double* __restrict__ x) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) x[i] += d[i];
+// X += D (n x nrhs, D dense): one launch for all columns.
+__global__ void axpy_kernel(int64_t n, int64_t nrhs, const double* __restrict__ d,
+                            double* __restrict__ x, int64_t ldx) {
+  const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (e < n * nrhs) {
+    const int64_t c = e / n;
+    x[e - c * n + c * ldx] += d[e];
+  }
 }
 
 
-// ---- residuals of several right-hand sides: R = B - op(A) X, columns in
-// groups of kRG, A read once per group (fp64 arithmetic, each sum in a fixed
-// order, so the result does not depend on scheduling).  maxes[3c .. 3c+2]
-// receive max |r|, |x|, |b| of column c.
-constexpr int kRG = 8;    // right-hand sides per group
-constexpr int kRK = 64;   // rows of X staged per step (not transposed)
-
-__device__ __forceinline__ void atomic_max_abs(unsigned long long* p, double v) {
-  atomicMax(p, (unsigned long long)__double_as_longlong(fabs(v)));
+// ---- residuals of several right-hand sides: R = B - op(A) X on the FP64
+// matrix instruction.  A CTA of eight warps computes RG x 16 rows of R for 8 NF
+// right-hand sides; KS = 8 / RG warps share each 16 rows, each taking its 32 of
+// every 32 KS values of the sum.  A goes straight from global memory to
+// registers (fp32, converted there), one stage of 32 ahead; X is staged in
+// shared memory by cp.async.  The sums' order is fixed, so the result does
+// not depend on scheduling.  maxes[3c .. 3c+2] receive max |r|, |x|, |b| of
+// column c.
+//
+// Bound by the FP64 rate from 32 right-hand sides on (n = 8192, 64 columns: 4.3
+// G multiply-adds, 0.24 ms at 64 per cycle and SM), below that by reading A
+// once, for which KS grows as NF shrinks: more, smaller CTAs in flight.  n =
+// 8192, 64 columns on B200: 0.52 ms (transposed 0.47), against 1.20 (1.86)
+// with plain FMAs in groups of 8 columns.
+// Bit pattern of |v|: ordered like the values, NaN above infinity.
+__device__ __forceinline__ unsigned long long abs_bits(double v) {
+  return (unsigned long long)__double_as_longlong(fabs(v));
 }
 
-// Not transposed: thread per row i, sums over k in order.
+constexpr int kRK = 32;   // values of a sum per warp and stage
+
+template <int NF, int KS>
+constexpr size_t residual_smem() {
+  return (size_t)2 * 8 * NF * (kRK * KS + 4) * sizeof(double);
+}
+
+template <bool TRANS, int NF, int KS>
 __global__ void __launch_bounds__(kT)
 residual_multi_kernel(int64_t n, int64_t nrhs, const float* __restrict__ A, int64_t lda,
                       const double* __restrict__ B, int64_t ldb,
                       const double* __restrict__ X, int64_t ldx, double* __restrict__ R,
                       int64_t ldr, unsigned long long* __restrict__ maxes) {
-  __shared__ double xs[kRK][kRG];
-  const int tid = threadIdx.x, lane = tid & 31;
-  const int64_t i = (int64_t)blockIdx.x * kT + tid;
-  const int64_t c0 = (int64_t)blockIdx.y * kRG;
-  const int nc = (int)((nrhs - c0) < kRG ? (nrhs - c0) : kRG);
-  double acc[kRG];
+  constexpr int RG = 8 / KS, NC = 8 * NF, KT = kRK * KS;
+  constexpr int S = KT + 4;   // column stride of the X stage: conflict-free fragment reads
+  extern __shared__ __align__(16) double xs[];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int rg = warp % RG, kh = warp / RG, lr = lane >> 2, lk = lane & 3;
+  const int64_t r0 = ((int64_t)blockIdx.x * RG + rg) * 16;
+  const int64_t c0 = (int64_t)blockIdx.y * NC;
+  const int nc = (int)((nrhs - c0) < NC ? (nrhs - c0) : NC);
+
+  // op(A) rows r0 + lr and r0 + 8 + lr; rows past n repeat the last one (their
+  // sums are dropped)
+  const float* arow[2];
 #pragma unroll
-  for (int c = 0; c < kRG; ++c) acc[c] = 0.0;
-  const float* row = A + (i < n ? i : 0);
-  for (int64_t k0 = 0; k0 < n; k0 += kRK) {
-    const int kw = (int)((n - k0) < kRK ? (n - k0) : kRK);
-    for (int e = tid; e < kRK * kRG; e += kT) {
-      const int c = e / kRK, kk = e % kRK;
-      xs[kk][c] = (kk < kw && c < nc) ? X[(k0 + kk) + (c0 + c) * ldx] : 0.0;
-    }
-    __syncthreads();
-    if (i < n) {
-      if (kw == kRK) {
-#pragma unroll 8
-        for (int kk = 0; kk < kRK; ++kk) {
-          const double a = (double)row[(k0 + kk) * lda];
+  for (int m = 0; m < 2; ++m) {
+    const int64_t r = r0 + 8 * m + lr < n ? r0 + 8 * m + lr : n - 1;
+    arow[m] = TRANS ? A + r * lda : A + r;
+  }
+  const bool vec = TRANS && ((reinterpret_cast<uintptr_t>(A) & 7) == 0) && (lda & 1) == 0;
+  // entry s of a stage: this lane's k = 4 s + lk, or (transposed) 8 (s / 2) + 2
+  // lk + (s & 1), so that a lane reads neighbours; k past n repeats the last
+  // one against zeros of X
+  auto load_a = [&](int64_t kb, float (&v)[8][2]) {
 #pragma unroll
-          for (int c = 0; c < kRG; ++c) acc[c] = fma(a, xs[kk][c], acc[c]);
-        }
-      } else {
-        for (int kk = 0; kk < kw; ++kk) {
-          const double a = (double)row[(k0 + kk) * lda];
+    for (int s = 0; s < 8; s += TRANS ? 2 : 1)
 #pragma unroll
-          for (int c = 0; c < kRG; ++c) acc[c] = fma(a, xs[kk][c], acc[c]);
+      for (int m = 0; m < 2; ++m) {
+        if (TRANS) {
+          const int64_t k = kb + 4 * s + 2 * lk;
+          if (vec && k + 1 < n) {
+            const float2 y = *reinterpret_cast<const float2*>(arow[m] + k);
+            v[s][m] = y.x;
+            v[s + 1][m] = y.y;
+          } else {
+            v[s][m] = arow[m][k < n ? k : n - 1];
+            v[s + 1][m] = arow[m][k + 1 < n ? k + 1 : n - 1];
+          }
+        } else {
+          const int64_t k = kb + 4 * s + lk;
+          v[s][m] = arow[m][(k < n ? k : n - 1) * lda];
         }
       }
+  };
+  auto load_x = [&](int64_t k0, double* dst) {
+    for (int e = tid; e < NC * KT; e += kT) {
+      const int c = e / KT, k = e % KT;
+      const bool ok = c < nc && k0 + k < n;
+      const double* src = ok ? X + (k0 + k) + (c0 + c) * ldx : X;
+      const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(dst + c * S + k));
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src),
+                   "r"(ok ? 8 : 0) : "memory");
+    }
+    trsv::cp_commit();
+  };
+
+  double acc[2][NF][2];
+#pragma unroll
+  for (int m = 0; m < 2; ++m)
+#pragma unroll
+    for (int f = 0; f < NF; ++f) acc[m][f][0] = acc[m][f][1] = 0.0;
+  float cur[8][2], nxt[8][2];
+  load_x(0, xs);
+  load_a(kRK * kh, cur);
+  const int nst = (int)((n + KT - 1) / KT);
+#pragma unroll 1
+  for (int t = 0; t < nst; ++t) {
+    const int64_t k1 = (int64_t)(t + 1) * KT;
+    trsv::cp_wait<0>();
+    __syncthreads();  // stage t is in, stage t - 1 read
+    if (t + 1 < nst) {
+      load_x(k1, xs + ((t + 1) & 1) * NC * S);
+      load_a(k1 + kRK * kh, nxt);
+    }
+    const double* x = xs + (t & 1) * NC * S + lr * S + kRK * kh;
+#pragma unroll
+    for (int s = 0; s < 8; ++s) {
+      const int k = TRANS ? 8 * (s >> 1) + 2 * lk + (s & 1) : 4 * s + lk;
+      const double a0 = (double)cur[s][0], a1 = (double)cur[s][1];
+#pragma unroll
+      for (int f = 0; f < NF; ++f) {
+        const double b = x[8 * f * S + k];
+        mma64(acc[0][f], a0, b);
+        mma64(acc[1][f], a1, b);
+      }
+    }
+#pragma unroll
+    for (int s = 0; s < 8; ++s) {
+      cur[s][0] = nxt[s][0];
+      cur[s][1] = nxt[s][1];
+    }
+  }
+  // the KS partial sums of each row group, added in order
+  if (KS > 1) {
+    __syncthreads();
+    double* part = xs + ((size_t)(kh > 0 ? kh - 1 : 0) * RG + rg) * 32 * 4 * NF;
+    if (kh > 0) {
+#pragma unroll
+      for (int m = 0; m < 2; ++m)
+#pragma unroll
+        for (int f = 0; f < NF; ++f)
+#pragma unroll
+          for (int h = 0; h < 2; ++h) part[((m * NF + f) * 2 + h) * 32 + lane] = acc[m][f][h];
     }
     __syncthreads();
-  }
+    if (kh > 0) return;
+    for (int q = 0; q < KS - 1; ++q) {
+      const double* p = xs + ((size_t)q * RG + rg) * 32 * 4 * NF;
 #pragma unroll
-  for (int c = 0; c < kRG; ++c) {
-    double r = 0.0, x = 0.0, b = 0.0;
-    if (i < n && c < nc) {
-      b = B[i + (c0 + c) * ldb];
-      x = X[i + (c0 + c) * ldx];
-      r = b - acc[c];
-      R[i + (c0 + c) * ldr] = r;
-    }
-    double m[3] = {fabs(r), fabs(x), fabs(b)};
+      for (int m = 0; m < 2; ++m)
 #pragma unroll
-    for (int q = 0; q < 3; ++q) {
+        for (int f = 0; f < NF; ++f)
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) m[q] = fmax(m[q], __shfl_xor_sync(0xffffffffu, m[q], o));
-      if (lane == 0 && c < nc) atomic_max_abs(&maxes[3 * (c0 + c) + q], m[q]);
+          for (int h = 0; h < 2; ++h) acc[m][f][h] += p[((m * NF + f) * 2 + h) * 32 + lane];
     }
   }
+#pragma unroll
+  for (int f = 0; f < NF; ++f)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int c = 8 * f + 2 * lk + h;
+      unsigned long long m[3] = {0ull, 0ull, 0ull};
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const int64_t i = r0 + 8 * q + lr;
+        if (i < n && c < nc) {
+          const double b = B[i + (c0 + c) * ldb], x = X[i + (c0 + c) * ldx];
+          const double r = b - acc[q][f][h];
+          R[i + (c0 + c) * ldr] = r;
+          m[0] = max(m[0], abs_bits(r));
+          m[1] = max(m[1], abs_bits(x));
+          m[2] = max(m[2], abs_bits(b));
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+#pragma unroll
+        for (int o = 16; o >= 4; o >>= 1)
+          m[q] = max(m[q], __shfl_xor_sync(0xffffffffu, m[q], o));
+        if (lr == 0 && c < nc) atomicMax(&maxes[3 * (c0 + c) + q], m[q]);
+      }
+    }
 }
 
-// Transposed: r_j = b_j - sum_i A[i, j] x_i.  Warp w of a CTA owns columns
-// j0 + 4w .. j0 + 4w + 3 of A; lanes run over i (coalesced), each lane sums
-// its rows in order, then a halving exchange over the 32 lanes leaves the
-// (column, right-hand side) pair 4-column x 8-rhs index `lane` in lane.
-constexpr int kTJ = 4;                 // columns of A per warp
-constexpr int kTI = 256;               // rows of X staged per step
-__global__ void __launch_bounds__(kT)
-residual_multi_t_kernel(int64_t n, int64_t nrhs, const float* __restrict__ A, int64_t lda,
-                        const double* __restrict__ B, int64_t ldb,
-                        const double* __restrict__ X, int64_t ldx, double* __restrict__ R,
-                        int64_t ldr, unsigned long long* __restrict__ maxes) {
-  __shared__ double xs[kRG][kTI];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int64_t jb = (int64_t)blockIdx.x * (kT / 32) * kTJ + warp * kTJ;
-  const int64_t c0 = (int64_t)blockIdx.y * kRG;
-  const int nc = (int)((nrhs - c0) < kRG ? (nrhs - c0) : kRG);
-  double v[kTJ * kRG];
-#pragma unroll
-  for (int q = 0; q < kTJ * kRG; ++q) v[q] = 0.0;
-  for (int64_t i0 = 0; i0 < n; i0 += kTI) {
-    const int iw = (int)((n - i0) < kTI ? (n - i0) : kTI);
-    for (int e = tid; e < kTI * kRG; e += kT) {
-      const int c = e / kTI, ii = e % kTI;
-      xs[c][ii] = (ii < iw && c < nc) ? X[(i0 + ii) + (c0 + c) * ldx] : 0.0;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int jj = 0; jj < kTJ; ++jj) {
-      const int64_t j = jb + jj;
-      if (j < n) {
-        const float* col = A + j * lda + i0;
-        for (int ii = lane; ii < iw; ii += 32) {
-          const double a = (double)col[ii];
-#pragma unroll
-          for (int c = 0; c < kRG; ++c) v[jj * kRG + c] = fma(a, xs[c][ii], v[jj * kRG + c]);
-        }
-      }
-    }
-    __syncthreads();
-  }
-  // halving exchange: after the step with offset s, slot q holds index
-  // q + (bits of lane above s) -- finally slot 0 holds index `lane`
-#pragma unroll
-  for (int s = 16; s >= 1; s >>= 1) {
-    const bool up = lane & s;
-#pragma unroll
-    for (int q = 0; q < s; ++q) {
-      const double send = up ? v[q] : v[q + s];
-      const double keep = up ? v[q + s] : v[q];
-      v[q] = keep + __shfl_xor_sync(0xffffffffu, send, s);
-    }
-  }
-  const int jj = lane / kRG, c = lane % kRG;
-  const int64_t j = jb + jj;
-  if (j < n && c < nc) {
-    const double b = B[j + (c0 + c) * ldb];
-    const double x = X[j + (c0 + c) * ldx];
-    const double r = b - v[0];
-    R[j + (c0 + c) * ldr] = r;
-    atomic_max_abs(&maxes[3 * (c0 + c)], r);
-    atomic_max_abs(&maxes[3 * (c0 + c) + 1], x);
-    atomic_max_abs(&maxes[3 * (c0 + c) + 2], b);
-  }
+template <bool TRANS, int NF, int KS>
+lu_status launch_residual_as(cudaStream_t st, int64_t n, int64_t nrhs, const float* A,
+                             int64_t lda, const double* B, int64_t ldb, const double* X,
+                             int64_t ldx, double* R, int64_t ldr, unsigned long long* maxes) {
+  const int64_t groups = ceil_div(nrhs, 8 * NF);
+  if (groups > 65535) return LU_ERR_INVALID_ARG;
+  dim3 g((unsigned)ceil_div(n, 16 * (8 / KS)), (unsigned)groups);
+  LUB_CUDA_TRY(set_smem_limit((const void*)residual_multi_kernel<TRANS, NF, KS>,
+                              residual_smem<NF, KS>()));
+  residual_multi_kernel<TRANS, NF, KS><<<g, kT, residual_smem<NF, KS>(), st>>>(
+      n, nrhs, A, lda, B, ldb, X, ldx, R, ldr, maxes);
+  LUB_LAUNCH_CHECK();
+  return LU_SUCCESS;
+}
+
+// Right-hand sides per CTA: A is read once per group of columns.
+template <bool TRANS>
+lu_status launch_residual_nf(cudaStream_t st, int64_t n, int64_t nrhs, const float* A,
+                             int64_t lda, const double* B, int64_t ldb, const double* X,
+                             int64_t ldx, double* R, int64_t ldr, unsigned long long* maxes) {
+  const auto fn = nrhs <= 8    ? launch_residual_as<TRANS, 1, 8>
+                  : nrhs <= 16 ? launch_residual_as<TRANS, 2, 8>
+                  : nrhs <= 32 ? launch_residual_as<TRANS, 4, 4>
+                               : launch_residual_as<TRANS, 8, 2>;
+  return fn(st, n, nrhs, A, lda, B, ldb, X, ldx, R, ldr, maxes);
 }
 }  // namespace
 
@@ -1175,21 +1246,14 @@ lu_status launch_residual_multi(cudaStream_t st, int64_t n, int64_t nrhs, const 
                                 unsigned long long* maxes) {
   if (n <= 0 || nrhs <= 0) return LU_SUCCESS;
   LUB_CUDA_TRY(cudaMemsetAsync(maxes, 0, (size_t)3 * nrhs * sizeof(unsigned long long), st));
-  const int64_t groups = ceil_div(nrhs, kRG);
-  if (groups > 65535) return LU_ERR_INVALID_ARG;
-  if (!trans) {
-    dim3 g((unsigned)ceil_div(n, kT), (unsigned)groups);
-    residual_multi_kernel<<<g, kT, 0, st>>>(n, nrhs, A, lda, B, ldb, X, ldx, R, ldr, maxes);
-  } else {
-    dim3 g((unsigned)ceil_div(n, (kT / 32) * kTJ), (unsigned)groups);
-    residual_multi_t_kernel<<<g, kT, 0, st>>>(n, nrhs, A, lda, B, ldb, X, ldx, R, ldr, maxes);
-  }
-  LUB_LAUNCH_CHECK();
-  return LU_SUCCESS;
+  return trans ? launch_residual_nf<true>(st, n, nrhs, A, lda, B, ldb, X, ldx, R, ldr, maxes)
+               : launch_residual_nf<false>(st, n, nrhs, A, lda, B, ldb, X, ldx, R, ldr, maxes);
 }
 
-lu_status launch_axpy(cudaStream_t st, int64_t n, const double* d, double* x) {
-  axpy_kernel<<<(unsigned)ceil_div(n, 256), 256, 0, st>>>(n, d, x);
+lu_status launch_axpy(cudaStream_t st, int64_t n, int64_t nrhs, const double* d, double* x,
+                      int64_t ldx) {
+  if (n <= 0 || nrhs <= 0) return LU_SUCCESS;
+  axpy_kernel<<<(unsigned)ceil_div(n * nrhs, 256), 256, 0, st>>>(n, nrhs, d, x, ldx);
   LUB_LAUNCH_CHECK();
   return LU_SUCCESS;
 }

@@ -47,7 +47,8 @@ lu_status launch_residual_multi(cudaStream_t st, int64_t n, int64_t nrhs, const 
                                 unsigned long long* maxes);
 
 // x += d
-lu_status launch_axpy(cudaStream_t st, int64_t n, const double* d, double* x);
+lu_status launch_axpy(cudaStream_t st, int64_t n, int64_t nrhs, const double* d, double* x,
+                      int64_t ldx);
 
 // adjoint.cu: dA = alpha * P Q^T (fp64 in, fp32 out); r = b - A^T x; ||A||_1
 lu_status launch_outer(cudaStream_t st, int64_t n, int64_t k, double alpha,
