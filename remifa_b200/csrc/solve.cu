@@ -10,25 +10,30 @@
 // factorization error -- what iterative refinement in fp64 needs.
 //
 // op(T) X = B, T = L (unit lower) or U (upper), op = identity or transpose,
-// runs as one launch per triangle (trsv_kernel) after a copy kernel that
-// moves B aside and marks every entry of X pending (a signalling-NaN
-// pattern no arithmetic produces).  A CTA per (row block of 64 rows, group
-// of up to 8 right-hand sides); CTAs draw tickets in solve order (an atomic
-// counter), so a CTA only ever waits for CTAs already running: no deadlock
-// whatever the residency.  Each warp of a CTA owns 8 rows of the block and
-// streams its share of the tiles op(T)[t, q] of the blocks solved earlier
-// through its own cp.async ring, reading the solution entries it needs
-// straight from X (relaxed loads at GPU scope, re-read while pending; the
-// solution IS the flag, so publishing a block costs one store, no fence and
-// no counter).  The diagonal block is inverted in fp64 and the last tile is
-// folded into W = Dinv op(T)[t, t-1] while the CTA waits, so the hand-over
-// from block t-1 to block t is, per warp and without a CTA barrier:
-// x_t = Dinv (b - sum_{q<t-1} op(T)[t,q] x_q) - W x_{t-1}, i.e. 16 fma per
-// lane and one shuffle reduction after x_{t-1} lands.
+// runs as one launch per triangle after a copy kernel that moves B aside and
+// marks every entry of X pending (a signalling-NaN pattern no arithmetic
+// produces).  A CTA per (row block of 64 rows, group of 1, 2 or 8 right-hand
+// sides); CTAs draw tickets in solve order (an atomic counter), so a CTA only
+// ever waits for CTAs already running: no deadlock whatever the residency.
+// Each warp of a CTA streams its share of the tiles op(T)[t, q] of the blocks
+// solved earlier, reading the solution entries it needs straight from X
+// (relaxed loads at GPU scope, re-read while pending; the solution IS the
+// flag, so publishing a block costs one store, no fence and no counter).  The
+// diagonal block is inverted in fp64 and the last tile is folded into W =
+// Dinv op(T)[t, t-1] while the CTA waits, so the hand-over from block t-1 to
+// block t is, per warp and without a CTA barrier: x_t = Dinv (b -
+// sum_{q<t-1} op(T)[t,q] x_q) - W x_{t-1}.  trsv_kernel does this with FMAs
+// and shuffles for 1 or 2 right-hand sides, trsv_mma_kernel on the FP64 matrix
+// instruction for groups of 8.  On B200: one right-hand side, n = 10007, L and U
+// 0.293 ms (0.344 without clusters), n = 16384 0.475 (0.573); 64 right-hand
+// sides, n = 8192 0.82 (1.36 with a counter per group and shared-memory
+// tiles).  Bound by the chain of n / 64 hand-overs.
 #include "common.cuh"
 #include "kernels.cuh"
 #include "mma64.cuh"
 #include "solve.cuh"
+
+#include <atomic>
 
 namespace lub {
 namespace {
@@ -46,14 +51,13 @@ struct Args {
   int64_t ld;
   double* X;        // solutions, written in place
   int64_t ldx;
-  const double* B;  // right-hand sides (n x nrhs, ld n) of the warp kernel
+  const double* B;  // right-hand sides (n x nrhs, ld n)
   int64_t n;
   int64_t nrhs;
   int nblk;
   int ngroups;
   int forward;      // op(T) lower: L or U^T
   int unit;         // unit diagonal: L or L^T
-  int xvec;         // X 16-byte aligned with even ldx (group kernel: cp.async)
   unsigned* sync;
   unsigned long long wait_ns;  // bound of one wait (kWaitNs)
   int withhold;     // self-test of the give-up path only: the row block solved
@@ -164,15 +168,37 @@ __device__ __forceinline__ void load_diag(float* dst, const Args& a, int64_t r0,
 // Inverse of the diagonal block of op(T) (fp32 in Dsrc as load_diag left it)
 // by fp64 substitution with the reciprocals of the diagonal: column j by
 // lanes 4j .. 4j+3, part p holding rows 4s + p.  Written row-major into
-// Dinv[r * 64 + j] (the same space as Dsrc; a barrier separates the reads
-// from the writes).  Rows and columns past rw are the identity.  All threads.
-template <bool TRANS>
+// Dinv[r * DS + j] (the same space as Dsrc; barriers separate the reads from
+// the writes).  The block is converted to fp64 once, in place (column k at Dinv
+// + 64 k): converting inside the substitution took most of its time.  Rows
+// and columns past rw are the identity.  All threads.
+template <bool TRANS, int DS = BS>
 __device__ __forceinline__ void invert_diag(const float* Dsrc, double* Dinv, double* rdiag,
                                             int rw, bool fwd, bool unit) {
   const int tid = threadIdx.x, lane = tid & 31;
-  auto D = [&](int r, int k) -> double {
-    return (double)(TRANS ? Dsrc[r * BS + k] : Dsrc[k * BS + r]);
-  };
+  {
+    // thread: 4 x 4 elements of memory column 4 (tid / 16) + e, rows 4 (tid % 16) ..
+    float v[4][4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float4 u = *reinterpret_cast<const float4*>(Dsrc + (4 * (tid >> 4) + e) * BS +
+                                                        4 * (tid & 15));
+      v[e][0] = u.x; v[e][1] = u.y; v[e][2] = u.z; v[e][3] = u.w;
+    }
+    __syncthreads();
+    const int mc = 4 * (tid >> 4), mr = 4 * (tid & 15);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      // op(T) row r, column k at Dinv[k * 64 + r]
+      double* d = TRANS ? Dinv + (mr + e) * BS + mc : Dinv + (mc + e) * BS + mr;
+      *reinterpret_cast<double2*>(d) = TRANS ? make_double2(v[0][e], v[1][e])
+                                             : make_double2(v[e][0], v[e][1]);
+      *reinterpret_cast<double2*>(d + 2) = TRANS ? make_double2(v[2][e], v[3][e])
+                                                 : make_double2(v[e][2], v[e][3]);
+    }
+    __syncthreads();
+  }
+  auto D = [&](int r, int k) -> double { return Dinv[k * BS + r]; };
   if (tid < BS) rdiag[tid] = (unit || tid >= rw) ? 1.0 : 1.0 / D(tid, tid);
   __syncthreads();
   const int j = tid >> 2, p = tid & 3;
@@ -204,9 +230,9 @@ __device__ __forceinline__ void invert_diag(const float* Dsrc, double* Dinv, dou
       }
     }
   }
-  __syncthreads();  // every read of the fp32 block precedes the overwrite
+  __syncthreads();  // every read of the block precedes the overwrite
 #pragma unroll
-  for (int s = 0; s < 16; ++s) Dinv[(4 * s + p) * BS + j] = z[s];
+  for (int s = 0; s < 16; ++s) Dinv[(4 * s + p) * DS + j] = z[s];
   __syncthreads();
 }
 
@@ -245,6 +271,11 @@ __device__ __forceinline__ double row_reduce(double (&v)[8], int lane) {
 // ======================================================================
 
 constexpr int S = 3;                   // stages of each warp's tile ring
+// Row blocks solved one after another by the CTAs of one cluster: they hand
+// their solutions over through distributed shared memory (0.6 us a block on
+// B200, against 1.0 through L2 and 1.5 .. 2 from one cluster to the next, which
+// is why 16 rather than the portable 8).
+constexpr int kCluster = 16;
 constexpr int kWarpTile = 8 * BS;      // floats of a warp's share of a tile
 // Marks a solution entry not yet published: a signalling-NaN payload that no
 // arithmetic produces (published NaNs are stored as the canonical quiet NaN).
@@ -257,6 +288,7 @@ __host__ __device__ constexpr size_t warp_smem_bytes(int nr) {
          + (size_t)BS * BS * 4            // tile of the previous block (fp32)
          + (size_t)8 * nr * BS * 8        // per-warp partial sums
          + (size_t)BS * 8                 // reciprocals of the diagonal
+         + (size_t)kCluster * nr * BS * 8 // solutions of the cluster's blocks
          + 64;                            // control words
 }
 
@@ -265,11 +297,51 @@ __device__ __forceinline__ double ld_poll(const double* p) {
   asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
   return __longlong_as_double((long long)v);
 }
+__device__ __forceinline__ unsigned long long publish_bits(double x) {
+  const unsigned long long v = (unsigned long long)__double_as_longlong(x);
+  return (v & 0x7ff0000000000000ull) == 0x7ff0000000000000ull && (v & 0xfffffffffffffull)
+             ? kQuietNaN : v;
+}
 __device__ __forceinline__ void st_publish(double* p, double x) {
-  unsigned long long v = (unsigned long long)__double_as_longlong(x);
-  if ((v & 0x7ff0000000000000ull) == 0x7ff0000000000000ull && (v & 0xfffffffffffffull))
-    v = kQuietNaN;
+  const unsigned long long v = publish_bits(x);
   asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+// Distributed shared memory: the cluster barrier, this CTA's rank, 8-byte and
+// 4-byte stores to the same place in another CTA of the cluster.
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\t"
+               "barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ int cluster_rank() {
+  unsigned r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return (int)r;
+}
+__device__ __forceinline__ uint32_t map_rank(const void* p, int rank) {
+  const uint32_t a = static_cast<uint32_t>(__cvta_generic_to_shared(p));
+  uint32_t d;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(rank));
+  return d;
+}
+__device__ __forceinline__ void st_remote64(const double* p, int rank, unsigned long long v) {
+  asm volatile("st.relaxed.cluster.shared::cluster.b64 [%0], %1;" ::"r"(map_rank(p, rank)), "l"(v)
+               : "memory");
+}
+__device__ __forceinline__ void st_remote32(const int* p, int rank, int v) {
+  asm volatile("st.relaxed.cluster.shared::cluster.b32 [%0], %1;" ::"r"(map_rank(p, rank)), "r"(v)
+               : "memory");
+}
+__device__ __forceinline__ double ld_local64(const double* p) {
+  unsigned long long v;
+  asm volatile("ld.relaxed.cluster.shared::cta.b64 %0, [%1];"
+               : "=l"(v) : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(p))) : "memory");
+  return __longlong_as_double((long long)v);
+}
+__device__ __forceinline__ int ld_local32(const int* p) {
+  int v;
+  asm volatile("ld.relaxed.cluster.shared::cta.b32 %0, [%1];"
+               : "=r"(v) : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(p))) : "memory");
+  return v;
 }
 __device__ __forceinline__ bool pending(double x) {
   return (unsigned long long)__double_as_longlong(x) == kPending;
@@ -372,6 +444,75 @@ __device__ __forceinline__ void settle_x(double (&x)[NX][NR], const Args& a, int
   }
 }
 
+// The same entries of a block that a CTA of this cluster solves, from the copy it
+// writes into this CTA's shared memory (xin: [column][row]); the wait bounded
+// as in settle_x.
+template <int NX, int NR>
+__device__ __forceinline__ void settle_local(double (&x)[NX][NR], const Args& a,
+                                             const double* xin, int kw, int nc, int kb, int ks,
+                                             int lane) {
+#pragma unroll
+  for (int h = 0; h < NX; ++h)
+#pragma unroll
+    for (int c = 0; c < NR; ++c)
+      x[h][c] = (kb + h * ks < kw && c < nc) ? __longlong_as_double((long long)kPending) : 0.0;
+  unsigned long long t0 = 0;
+  for (unsigned it = 0;; ++it) {
+    bool ok = true;
+#pragma unroll
+    for (int h = 0; h < NX; ++h)
+#pragma unroll
+      for (int c = 0; c < NR; ++c)
+        if (pending(x[h][c])) {
+          x[h][c] = ld_local64(xin + c * BS + kb + h * ks);
+          ok &= !pending(x[h][c]);
+        }
+    if (__all_sync(0xffffffffu, ok)) return;
+    if ((it & 31u) != 31u) continue;
+    const unsigned long long now = global_ns();
+    if (t0 == 0) t0 = now;
+    const bool expired = now - t0 > a.wait_ns;
+    if (__any_sync(0xffffffffu, expired || *(volatile unsigned*)(a.sync + 1) != 0u)) {
+#pragma unroll
+      for (int h = 0; h < NX; ++h)
+#pragma unroll
+        for (int c = 0; c < NR; ++c)
+          if (pending(x[h][c])) x[h][c] = __longlong_as_double((long long)kQuietNaN);
+      if (lane == 0 && expired) atomicAdd(a.sync + 1, 1u);
+      return;
+    }
+  }
+}
+
+// settle_x for the matrix kernel's hand-over: entry e is row 8 (e / 2) + 2 lk +
+// (e & 1) of one column.
+__device__ __forceinline__ void settle_mma(double (&x)[16][1], const Args& a, int64_t k0,
+                                           int64_t c, int lk, int lane) {
+  bool ok = true;
+#pragma unroll
+  for (int e = 0; e < 16; ++e) ok &= !pending(x[e][0]);
+  if (__all_sync(0xffffffffu, ok)) return;
+  const unsigned long long t0 = global_ns();
+  for (;;) {
+    ok = true;
+#pragma unroll
+    for (int e = 0; e < 16; ++e)
+      if (pending(x[e][0])) {
+        x[e][0] = ld_poll(a.X + k0 + 8 * (e >> 1) + 2 * lk + (e & 1) + c * a.ldx);
+        ok &= !pending(x[e][0]);
+      }
+    if (__all_sync(0xffffffffu, ok)) return;
+    const bool expired = global_ns() - t0 > a.wait_ns;
+    if (__any_sync(0xffffffffu, expired || *(volatile unsigned*)(a.sync + 1) != 0u)) {
+#pragma unroll
+      for (int e = 0; e < 16; ++e)
+        if (pending(x[e][0])) x[e][0] = __longlong_as_double((long long)kQuietNaN);
+      if (lane == 0 && expired) atomicAdd(a.sync + 1, 1u);
+      return;
+    }
+  }
+}
+
 // One CTA per (row block, group): warps stream their shares of the tiles
 // of all blocks but the previous one without CTA barriers; one barrier
 // combines the partial sums into c = Dinv y; the hand-over x = c - W x_prev
@@ -388,13 +529,37 @@ trsv_kernel(Args a) {
   float* Tw = reinterpret_cast<float*>(Dinv + BS * BS);
   double* part = reinterpret_cast<double*>(Tw + BS * BS);
   double* rdiag = part + 8 * NR * BS;
-  int* ctrl = reinterpret_cast<int*>(rdiag + BS);
+  double* xin = rdiag + BS;              // [block of the cluster][column][row]
+  int* ctrl = reinterpret_cast<int*>(xin + kCluster * NR * BS);
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid == 0) ctrl[0] = (int)atomicAdd(a.sync, 1u);
+  // the cluster's ticket: its kCluster consecutive row blocks of one group
+  const int rank = cluster_rank();
+  for (int e = tid; e < kCluster * NR * BS; e += kThreads)
+    xin[e] = __longlong_as_double((long long)kPending);
+  if (tid == 0) ctrl[0] = -1;
+  cluster_sync();   // every CTA runs and has its markers in place
+  if (rank == 0 && tid < kCluster) {
+    int tk = 0;
+    if (tid == 0) tk = (int)atomicAdd(a.sync, 1u);
+    tk = __shfl_sync((1u << kCluster) - 1, tk, 0);
+    st_remote32(ctrl, tid, tk);
+  }
+  if (tid == 0) {
+    // the store is on its way; bounded like every wait
+    int tk = -1;
+    for (int it = 0; it < (1 << 24) && tk < 0; ++it) tk = ld_local32(ctrl);
+    if (tk < 0) atomicAdd(a.sync + 1, 1u);
+    ctrl[1] = tk;
+  }
   __syncthreads();
-  const int ticket = ctrl[0];
-  const int t = ticket / a.ngroups, g = ticket - t * a.ngroups;
+  const int ticket = ctrl[1];
+  const int base = ticket / a.ngroups * kCluster;     // first block of the cluster
+  const int t = base + rank, g = ticket % a.ngroups;
+  if (ticket < 0 || t >= a.nblk) {
+    cluster_sync();   // as at the end
+    return;
+  }
   const bool fwd = a.forward != 0;
   const int64_t r0 = (int64_t)(fwd ? t : a.nblk - 1 - t) * BS;
   const int rw = imin64(a.n - r0, BS);
@@ -403,6 +568,7 @@ trsv_kernel(Args a) {
   auto tile_k0 = [&](int q) -> int64_t { return (int64_t)(fwd ? q : a.nblk - 1 - q) * BS; };
   auto tile_kw = [&](int q) -> int { return imin64(a.n - tile_k0(q), BS); };
   const int nbulk = t > 1 ? t - 1 : 0;  // tiles before the previous block's
+  const int nglob = nbulk < base ? nbulk : base;  // of them, solved by other clusters
   // tile columns whose solution entries this lane reads in the bulk phase
   const int kb = TRANS ? lane : 8 * warp + (lane & 7);
   const int ks = TRANS ? 32 : 0;
@@ -424,7 +590,7 @@ trsv_kernel(Args a) {
   double xq[PD][NX][NR];
 #pragma unroll
   for (int d = 0; d < PD; ++d)
-    if (d < nbulk) fetch_x<NX, NR>(xq[d], a, tile_k0(d), tile_kw(d), c0, nc, kb, ks);
+    if (d < nglob) fetch_x<NX, NR>(xq[d], a, tile_k0(d), tile_kw(d), c0, nc, kb, ks);
   // right-hand sides of rows lane and lane + 32
   double bm[2][NR];
 #pragma unroll
@@ -493,9 +659,10 @@ trsv_kernel(Args a) {
       for (int h = 0; h < NX; ++h)
 #pragma unroll
         for (int c = 0; c < NR; ++c) xq[d][h][c] = xq[d + 1][h][c];
-    if (q + PD < nbulk)
+    if (q + PD < nglob)
       fetch_x<NX, NR>(xq[PD - 1], a, tile_k0(q + PD), tile_kw(q + PD), c0, nc, kb, ks);
-    settle_x<NX, NR>(x, a, tile_k0(q), c0, kb, ks, lane);
+    if (q < nglob) settle_x<NX, NR>(x, a, tile_k0(q), c0, kb, ks, lane);
+    else settle_local<NX, NR>(x, a, xin + (q - base) * NR * BS, tile_kw(q), nc, kb, ks, lane);
     cp_wait<S - 2>();
     __syncwarp();
     issue(q + S - 1);
@@ -530,7 +697,8 @@ trsv_kernel(Args a) {
 
   // the previous block's solution: fetched now, waited for after c
   double xf[2][NR];
-  if (t >= 1) fetch_x<2, NR>(xf, a, tile_k0(t - 1), tile_kw(t - 1), c0, nc, lane, 32);
+  if (t >= 1 && rank == 0)
+    fetch_x<2, NR>(xf, a, tile_k0(t - 1), tile_kw(t - 1), c0, nc, lane, 32);
 
   // ---- partial sums of the warps -> y = b - sum -> c = Dinv y ----
   if (TRANS) {
@@ -576,7 +744,8 @@ trsv_kernel(Args a) {
 
   // ---- hand-over: x = c - W x_prev once the previous block is out ----
   if (t >= 1) {
-    settle_x<2, NR>(xf, a, tile_k0(t - 1), c0, lane, 32, lane);
+    if (rank == 0) settle_x<2, NR>(xf, a, tile_k0(t - 1), c0, lane, 32, lane);
+    else settle_local<2, NR>(xf, a, xin + (rank - 1) * NR * BS, tile_kw(t - 1), nc, lane, 32, lane);
 #pragma unroll
     for (int c = 0; c < NR; ++c) {
       double v[8];
@@ -585,12 +754,24 @@ trsv_kernel(Args a) {
       cv[c] -= row_reduce(v, lane);
     }
   }
+  // to the later CTAs of the cluster (a row's four lanes take turns), then to
+  // the other clusters
   const int ri = 8 * warp + (lane >> 2);
-  if ((lane & 3) == 0 && ri < rw && ticket != a.withhold) {
+  if (ri < rw && t != a.withhold) {
 #pragma unroll
     for (int c = 0; c < NR; ++c)
-      if (c < nc) st_publish(a.X + (r0 + ri) + (c0 + c) * a.ldx, cv[c]);
+      if (c < nc) {
+#pragma unroll
+        for (int h = 0; h < kCluster / 4; ++h) {
+          const int to = rank + 1 + (lane & 3) + 4 * h;
+          if (to < kCluster && base + to < a.nblk)
+            st_remote64(xin + (rank * NR + c) * BS + ri, to, publish_bits(cv[c]));
+        }
+        if ((lane & 3) == 0) st_publish(a.X + (r0 + ri) + (c0 + c) * a.ldx, cv[c]);
+      }
   }
+  // no CTA leaves while another may still write into its shared memory
+  cluster_sync();
 }
 
 // B <- X and X <- pending, for the rows and columns of the solve; the first
@@ -611,221 +792,209 @@ __global__ void trsv_prepare_kernel(int64_t n, int64_t nrhs, double* __restrict_
 }
 
 // ======================================================================
-// Group kernel (groups of 4 or 8 right-hand sides).  Row blocks publish
-// through a per-group counter of finished blocks (release / acquire at GPU
-// scope); the solution blocks of finished blocks are staged through the
-// CTA's cp.async ring together with the tiles, so a CTA that starts behind
-// the solve front streams its backlog at memory speed.
+// Matrix kernel (groups of 8 right-hand sides): the same scheme on mma64.
+// Warp w takes columns 8w .. 8w + 7 of every tile for all 64 rows -- each tile
+// element is loaded and converted once per CTA, straight from global memory to
+// registers one tile ahead, and a lane reads only two solution entries per
+// tile -- then rows 8w .. of Dinv y and of the hand-over.
+//
+// Bound by the FP64 rate (n = 8192, 64 right-hand sides: 2.1 G multiply-adds
+// per triangle, 0.12 ms) and, as long, by the chain of n / 64 hand-overs.
 // ======================================================================
 
-constexpr int kGS = 4;                 // ring stages of the group kernel
-constexpr int kSyncHeader = 4;         // ticket, abort, expired waits, spare
+constexpr int DS = BS + 4;   // row stride of Dinv: conflict-free fragment reads
+constexpr int YS = 12;       // row stride of y, likewise
+constexpr int kHeader = 4;   // words of the sync area: ticket, expired waits, spare
 
-__host__ __device__ constexpr size_t group_smem_bytes(int nr) {
-  return (size_t)kGS * BS * BS * 4        // fp32 tiles
-         + (size_t)kGS * nr * BS * 8      // fp64 solution blocks of the tiles
-         + (size_t)BS * BS * 8            // inverse of the diagonal block
-         + (size_t)nr * BS * 8            // right-hand side / y
-         + (size_t)BS * 8                 // reciprocals of the diagonal
-         + 64;                            // control words
-}
-
-__device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
-  unsigned v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-__device__ __forceinline__ void st_release(unsigned* p, unsigned v) {
-  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+constexpr size_t mma_smem_bytes() {
+  return (size_t)BS * DS * 8          // inverse of the diagonal block (fp64)
+         + (size_t)BS * BS * 4        // tile of the previous block (fp32)
+         + (size_t)8 * BS * 8 * 8     // the warps' partial sums
+         + (size_t)BS * YS * 8        // y
+         + (size_t)BS * 8             // reciprocals of the diagonal
+         + 64;                        // control words
 }
 
-// Solution block of a tile: rows k0 .. k0+kw of the group's columns, the
-// rest zero.  Async form: 16-byte copies through L2 (the block was written
-// by another SM; L1 is bypassed).  Sync form: L2 loads.
-template <int NR>
-__device__ __forceinline__ void load_x_async(double* dst, const Args& a, int64_t k0, int kw,
-                                             int64_t c0, int nc) {
-  for (int e = threadIdx.x; e < NR * BS / 2; e += kThreads) {
-    const int c = e / (BS / 2), k = 2 * (e % (BS / 2));
-    const int valid = c < nc ? min(2, max(0, kw - k)) : 0;
-    const double* src = valid ? a.X + (k0 + k) + (c0 + c) * a.ldx : a.X;
-    cp16z(dst + c * BS + k, src, valid * 8);
-  }
-}
-template <int NR>
-__device__ __forceinline__ void load_x_sync(double* dst, const Args& a, int64_t k0, int kw,
-                                            int64_t c0, int nc) {
-  for (int e = threadIdx.x; e < NR * BS; e += kThreads) {
-    const int c = e / BS, k = e % BS;
-    dst[e] = (c < nc && k < kw) ? __ldcg(a.X + (k0 + k) + (c0 + c) * a.ldx) : 0.0;
-  }
-}
-
-template <bool TRANS, int NR, bool V16>
-__global__ void __launch_bounds__(kThreads, 1)
-trsv_group_kernel(Args a) {
+template <bool TRANS, bool V16>
+__global__ void __launch_bounds__(kThreads, 2)
+trsv_mma_kernel(Args a) {
+  constexpr int PD = 3;     // tiles whose solution entries are fetched ahead
   extern __shared__ __align__(16) unsigned char smem[];
-  float* Tr = reinterpret_cast<float*>(smem);
-  double* Xr = reinterpret_cast<double*>(smem + (size_t)kGS * BS * BS * 4);
-  double* Dinv = Xr + kGS * NR * BS;
-  double* ybuf = Dinv + BS * BS;
-  double* rdiag = ybuf + NR * BS;
-  int* ctrl = reinterpret_cast<int*>(rdiag + BS);  // ticket, avail[2], give-up
+  double* Dinv = reinterpret_cast<double*>(smem);
+  float* Tw = reinterpret_cast<float*>(Dinv + BS * DS);
+  double* part = reinterpret_cast<double*>(Tw + BS * BS);
+  double* ybuf = part + 8 * BS * 8;
+  double* rdiag = ybuf + BS * YS;
+  int* ctrl = reinterpret_cast<int*>(rdiag + BS);
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  unsigned* abort_word = a.sync + 1;
-  if (tid == 0) {
-    const unsigned tk = atomicAdd(a.sync, 1u);
-    ctrl[0] = (int)tk;
-    ctrl[1] = (int)ld_acquire(a.sync + kSyncHeader + tk % (unsigned)a.ngroups);
-    ctrl[3] = 0;
-  }
+  const int lr = lane >> 2, lk = lane & 3;
+  if (tid == 0) ctrl[0] = (int)atomicAdd(a.sync, 1u);
   __syncthreads();
   const int ticket = ctrl[0];
   const int t = ticket / a.ngroups, g = ticket - t * a.ngroups;
   const bool fwd = a.forward != 0;
   const int64_t r0 = (int64_t)(fwd ? t : a.nblk - 1 - t) * BS;
   const int rw = imin64(a.n - r0, BS);
-  const int64_t c0 = (int64_t)g * NR;
-  const int nc = imin64(a.nrhs - c0, NR);
-  unsigned* done = a.sync + kSyncHeader + g;
+  const int64_t c0 = (int64_t)g * 8;
+  const int nc = imin64(a.nrhs - c0, 8);
   auto tile_k0 = [&](int q) -> int64_t { return (int64_t)(fwd ? q : a.nblk - 1 - q) * BS; };
   auto tile_kw = [&](int q) -> int { return imin64(a.n - tile_k0(q), BS); };
+  const int nbulk = t > 1 ? t - 1 : 0;  // tiles before the previous block's
 
-  // right-hand side rows of this block
-  for (int e = tid; e < NR * BS; e += kThreads) {
-    const int c = e / BS, r = e % BS;
-    ybuf[e] = (c < nc && r < rw) ? a.X[(r0 + r) + (c0 + c) * a.ldx] : 0.0;
-  }
+  // ---- set-up copies: diagonal block, previous block's tile
   float* Dsrc = reinterpret_cast<float*>(Dinv);
   load_diag<V16>(Dsrc, a, r0, rw);
+  if (t >= 1) load_tile<TRANS, V16>(Tw, a, r0, rw, tile_k0(t - 1), tile_kw(t - 1));
   cp_commit();
-  int avail = ctrl[1];
-  unsigned xbits = 0;
-  auto issue = [&](int q) {
-    if (q < t) {
-      const int st = q % kGS;
-      const int64_t k0 = tile_k0(q);
-      const int kw = tile_kw(q);
-      load_tile<TRANS, V16>(Tr + st * BS * BS, a, r0, rw, k0, kw);
-      if (a.xvec && q < avail) {
-        load_x_async<NR>(Xr + st * NR * BS, a, k0, kw, c0, nc);
-        xbits |= 1u << st;
+
+  // This warp's share of tile q: entry [m][s] is row 8 m + lr and column kk(s).
+  // Rows and columns past the matrix repeat the last one (their sums are
+  // dropped, or meet zeros of x).
+  auto kk = [&](int s) { return 8 * warp + (TRANS ? 2 * lk + s : 4 * s + lk); };
+  auto load_a = [&](int q, float (&v)[8][2]) {
+    const int64_t k0 = tile_k0(q);
+    const int kw = tile_kw(q);
+#pragma unroll
+    for (int m = 0; m < 8; ++m) {
+      const int64_t r = r0 + (8 * m + lr < rw ? 8 * m + lr : rw - 1);
+      if (TRANS && V16 && kw == BS) {
+        const float2 y = *reinterpret_cast<const float2*>(a.lu + k0 + kk(0) + r * a.ld);
+        v[m][0] = y.x;
+        v[m][1] = y.y;
       } else {
-        xbits &= ~(1u << st);
-      }
-    }
-    cp_commit();
-  };
-#pragma unroll 1
-  for (int q = 0; q < kGS - 1; ++q) issue(q);
-
-  cp_wait<kGS - 1>();
-  __syncthreads();
-  invert_diag<TRANS>(Dsrc, Dinv, rdiag, rw, fwd, a.unit != 0);
-
-  // ---- all tiles of the blocks solved before this one; warp w rows
-  // 8w .. 8w+7, per-lane partials over columns lane and lane + 32 ----
-  double acc[8][NR];
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
-#pragma unroll
-    for (int c = 0; c < NR; ++c) acc[i][c] = 0.0;
-  int refresh = 0;
-  bool aborted = false;
-#pragma unroll 1
-  for (int q = 0; q < t; ++q) {
-    if (q >= avail) {
-      // wait until solve position q is published (thread 0 polls, bounded)
-      if (tid == 0) {
-        unsigned v = ld_acquire(done);
-        if ((int)v <= q) {
-          const unsigned long long t0 = global_ns();
-          for (;;) {
-            v = ld_acquire(done);
-            if ((int)v > q) break;
-            if (*(volatile unsigned*)abort_word) { ctrl[3] = 1; break; }
-            if (global_ns() - t0 > a.wait_ns) {
-              atomicExch(abort_word, 1u);
-              atomicAdd(a.sync + 2, 1u);
-              ctrl[3] = 1;
-              break;
-            }
-          }
+        for (int s = 0; s < 2; ++s) {
+          const int64_t k = k0 + (kk(s) < kw ? kk(s) : kw - 1);
+          v[m][s] = TRANS ? a.lu[k + r * a.ld] : a.lu[r + k * a.ld];
         }
-        ctrl[1 + (refresh & 1)] = (int)v;
       }
-      __syncthreads();
-      avail = ctrl[1 + (refresh & 1)];
-      ++refresh;
-      if (ctrl[3]) { aborted = true; break; }
     }
-    const int st = q % kGS;
-    cp_wait<kGS - 2>();
-    if (!((xbits >> st) & 1u))
-      load_x_sync<NR>(Xr + st * NR * BS, a, tile_k0(q), tile_kw(q), c0, nc);
-    __syncthreads();
-    issue(q + kGS - 1);
-    const float* Ts = Tr + st * BS * BS;
-    const double* xs = Xr + st * NR * BS;
+  };
+  // Solution entries kb, kb + ks of column lr of the group, as loaded
+  const int xs = TRANS ? 1 : 4;
+  auto fetch = [&](double (&x)[2], int q) {
+    const int64_t k0 = tile_k0(q);
+    const int kw = tile_kw(q);
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int k = lane + 32 * h;
-      double xv[NR];
+    for (int s = 0; s < 2; ++s)
+      x[s] = (kk(s) < kw && lr < nc) ? ld_poll(a.X + k0 + kk(s) + (c0 + lr) * a.ldx) : 0.0;
+  };
+  float cur[8][2], nxt[8][2];
+  double xq[PD][2];
 #pragma unroll
-      for (int c = 0; c < NR; ++c) xv[c] = xs[c * BS + k];
-      float tv[8];
-      if (!TRANS) {
-        const float4 u0 = *reinterpret_cast<const float4*>(Ts + tile_index<false>(8 * warp, k));
-        const float4 u1 = *reinterpret_cast<const float4*>(Ts + tile_index<false>(8 * warp + 4, k));
-        tv[0] = u0.x; tv[1] = u0.y; tv[2] = u0.z; tv[3] = u0.w;
-        tv[4] = u1.x; tv[5] = u1.y; tv[6] = u1.z; tv[7] = u1.w;
-      } else {
+  for (int d = 0; d < PD; ++d)
+    if (d < nbulk) fetch(xq[d], d);
+  if (nbulk > 0) load_a(0, cur);
+  // right-hand side entries (row tid / 4, columns 2 (tid & 3) and the next)
+  double bm[2];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) tv[i] = Ts[tile_index<true>(8 * warp + i, k)];
-      }
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int c = 0; c < NR; ++c) acc[i][c] = fma((double)tv[i], xv[c], acc[i][c]);
-    }
+  for (int h = 0; h < 2; ++h) {
+    const int r = tid >> 2, c = 2 * (tid & 3) + h;
+    bm[h] = (r < rw && c < nc) ? a.B[(r0 + r) + (c0 + c) * a.n] : 0.0;
   }
   cp_wait<0>();
-  if (aborted) {
-    for (int e = tid; e < NR * BS; e += kThreads) {
-      const int c = e / BS, r = e % BS;
-      if (c < nc && r < rw)
-        a.X[(r0 + r) + (c0 + c) * a.ldx] = __longlong_as_double((long long)kQuietNaN);
+  __syncthreads();
+  invert_diag<TRANS, DS>(Dsrc, Dinv, rdiag, rw, fwd, a.unit != 0);
+
+  // ---- W = Dinv op(T)[block, previous block], rows 8 warp + lr: columns 8 f +
+  // 2 lk + h, which the hand-over takes as its k index
+  double W[8][2];
+#pragma unroll
+  for (int f = 0; f < 8; ++f) W[f][0] = W[f][1] = 0.0;
+  if (t >= 1) {
+#pragma unroll 2
+    for (int s = 0; s < BS / 4; ++s) {
+      const int k = 4 * s + lk;
+      const double d = Dinv[(8 * warp + lr) * DS + k];
+#pragma unroll
+      for (int f = 0; f < 8; ++f) mma64(W[f], d, (double)Tw[tile_index<TRANS>(k, 8 * f + lr)]);
     }
-    return;
   }
 
-  // ---- y = b - sum, then x = Dinv y (rows 8 warp + i, lanes over j) ----
+  // ---- bulk: the tiles before the previous block's
+  double acc[8][2];
 #pragma unroll
-  for (int c = 0; c < NR; ++c) {
-    double v[8];
+  for (int m = 0; m < 8; ++m) acc[m][0] = acc[m][1] = 0.0;
+#pragma unroll 1
+  for (int q = 0; q < nbulk; ++q) {
+    double x[2][1] = {{xq[0][0]}, {xq[0][1]}};
 #pragma unroll
-    for (int i = 0; i < 8; ++i) v[i] = acc[i][c];
-    const double s = row_reduce(v, lane);
-    if ((lane & 3) == 0) ybuf[c * BS + 8 * warp + (lane >> 2)] -= s;
+    for (int d = 0; d + 1 < PD; ++d) {
+      xq[d][0] = xq[d + 1][0];
+      xq[d][1] = xq[d + 1][1];
+    }
+    if (q + PD < nbulk) fetch(xq[PD - 1], q + PD);
+    if (q + 1 < nbulk) load_a(q + 1, nxt);
+    settle_x<2, 1>(x, a, tile_k0(q), c0 + lr, kk(0), xs, lane);
+#pragma unroll
+    for (int s = 0; s < 2; ++s)
+#pragma unroll
+      for (int m = 0; m < 8; ++m) mma64(acc[m], (double)cur[m][s], x[s][0]);
+#pragma unroll
+    for (int m = 0; m < 8; ++m) {
+      cur[m][0] = nxt[m][0];
+      cur[m][1] = nxt[m][1];
+    }
+  }
+
+  // the previous block's solution: fetched now, waited for after c
+  double xf[16][1];
+  if (t >= 1) {
+    const int64_t k0 = tile_k0(t - 1);
+    const int kw = tile_kw(t - 1);
+#pragma unroll
+    for (int e = 0; e < 16; ++e) {
+      const int k = 8 * (e >> 1) + 2 * lk + (e & 1);
+      xf[e][0] = (k < kw && lr < nc) ? ld_poll(a.X + k0 + k + (c0 + lr) * a.ldx) : 0.0;
+    }
+  }
+
+  // ---- partial sums of the warps -> y = b - sum -> c = Dinv y
+#pragma unroll
+  for (int m = 0; m < 8; ++m)
+    *reinterpret_cast<double2*>(part + (warp * BS + 8 * m + lr) * 8 + 2 * lk) =
+        make_double2(acc[m][0], acc[m][1]);
+  __syncthreads();
+  {
+    const int r = tid >> 2, c = 2 * (tid & 3);
+    double2 y = make_double2(0.0, 0.0);
+#pragma unroll
+    for (int w = 0; w < 8; ++w) {
+      const double2 p = *reinterpret_cast<const double2*>(part + (w * BS + r) * 8 + c);
+      y.x += p.x;
+      y.y += p.y;
+    }
+    // rows past the matrix stay zero
+    ybuf[r * YS + c] = r < rw ? bm[0] - y.x : 0.0;
+    ybuf[r * YS + c + 1] = r < rw ? bm[1] - y.y : 0.0;
   }
   __syncthreads();
-  const int ri = 8 * warp + (lane >> 2);
+  double cv[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
 #pragma unroll
-  for (int c = 0; c < NR; ++c) {
-    double v[8];
+  for (int s = 0; s < BS / 4; ++s)
+    mma64(cv[s & 1], Dinv[(8 * warp + lr) * DS + 4 * s + lk], ybuf[(4 * s + lk) * YS + lr]);
+  cv[0][0] += cv[1][0];
+  cv[0][1] += cv[1][1];
+
+  // ---- hand-over: x = c - W x_prev once the previous block is out
+  if (t >= 1) {
+    settle_mma(xf, a, tile_k0(t - 1), c0 + lr, lk, lane);
+    double h[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
-      v[i] = fma(Dinv[(8 * warp + i) * BS + lane + 32], ybuf[c * BS + lane + 32],
-                 Dinv[(8 * warp + i) * BS + lane] * ybuf[c * BS + lane]);
-    const double x = row_reduce(v, lane);
-    if ((lane & 3) == 0 && ri < rw && c < nc) a.X[(r0 + ri) + (c0 + c) * a.ldx] = x;
+    for (int e = 0; e < 16; ++e) mma64(h[e & 1], W[e >> 1][e & 1], xf[e][0]);
+    cv[0][0] -= h[0][0] + h[1][0];
+    cv[0][1] -= h[0][1] + h[1][1];
   }
-  __syncthreads();
-  if (tid == 0) st_release(done, (unsigned)(t + 1));
+  const int row = 8 * warp + lr;
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+    if (row < rw && 2 * lk + h < nc)
+      st_publish(a.X + (r0 + row) + (c0 + 2 * lk + h) * a.ldx, cv[0][h]);
 }
 
-int group_width(int64_t nrhs) { return nrhs >= 8 ? 8 : nrhs >= 4 ? 4 : nrhs >= 2 ? 2 : 1; }
+// Right-hand sides per CTA: from three on, the matrix kernel's 8.
+int group_width(int64_t nrhs) { return nrhs >= 3 ? 8 : nrhs == 2 ? 2 : 1; }
 
 template <bool TRANS, int NR, bool V16>
 lu_status launch_one(cudaStream_t st, const Args& a) {
@@ -834,12 +1003,35 @@ lu_status launch_one(cudaStream_t st, const Args& a) {
   if constexpr (NR <= 2) {
     smem = warp_smem_bytes(NR);
     fn = trsv_kernel<TRANS, NR, V16>;
+    LUB_CUDA_TRY(set_smem_limit((const void*)fn, smem));
+    // clusters of more than 8 CTAs are allowed per kernel, once per device
+    static std::atomic<uint64_t> allowed{0};
+    int dev = 0;
+    LUB_CUDA_TRY(cudaGetDevice(&dev));
+    const uint64_t bit = 1ull << (dev & 63);
+    if (!(allowed.load() & bit)) {
+      LUB_CUDA_TRY(cudaFuncSetAttribute((const void*)fn,
+                                        cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+      allowed.fetch_or(bit);
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(ceil_div(a.nblk, kCluster) * kCluster * a.ngroups));
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = kCluster;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    LUB_CUDA_TRY(cudaLaunchKernelEx(&cfg, fn, a));
   } else {
-    smem = group_smem_bytes(NR);
-    fn = trsv_group_kernel<TRANS, NR, V16>;
+    smem = mma_smem_bytes();
+    fn = trsv_mma_kernel<TRANS, V16>;
+    LUB_CUDA_TRY(set_smem_limit((const void*)fn, smem));
+    fn<<<(unsigned)((int64_t)a.nblk * a.ngroups), kThreads, smem, st>>>(a);
   }
-  LUB_CUDA_TRY(set_smem_limit((const void*)fn, smem));
-  fn<<<(unsigned)((int64_t)a.nblk * a.ngroups), kThreads, smem, st>>>(a);
   LUB_LAUNCH_CHECK();
   return LU_SUCCESS;
 }
@@ -848,7 +1040,6 @@ template <bool TRANS, bool V16>
 lu_status launch_nr(cudaStream_t st, const Args& a, int nr) {
   switch (nr) {
     case 8: return launch_one<TRANS, 8, V16>(st, a);
-    case 4: return launch_one<TRANS, 4, V16>(st, a);
     case 2: return launch_one<TRANS, 2, V16>(st, a);
     default: return launch_one<TRANS, 1, V16>(st, a);
   }
@@ -1149,8 +1340,8 @@ lu_status launch_residual_nf(cudaStream_t st, int64_t n, int64_t nrhs, const flo
 }  // namespace
 
 size_t trsm_sync_bytes(int64_t nrhs) {
-  const int64_t groups = ceil_div(nrhs < 1 ? 1 : nrhs, 4);
-  return align_up((size_t)(trsv::kSyncHeader + groups) * 4, 256);
+  (void)nrhs;
+  return align_up((size_t)trsv::kHeader * 4, 256);
 }
 
 size_t trsm_ws_bytes(int64_t n, int64_t nrhs) {
@@ -1179,18 +1370,13 @@ lu_status launch_trsm(cudaStream_t st, int64_t n, const float* lu, int64_t ld,
   // op(T) is lower (forward substitution) for L and for U^T
   a.forward = upper == trans;
   a.unit = !upper;
-  a.xvec = ((reinterpret_cast<uintptr_t>(X) & 15) == 0) && (ldx % 2 == 0);
   a.sync = sync;
   a.wait_ns = wait_ns > 0 ? wait_ns : trsv::kWaitNs;
   a.withhold = withhold;
-  if (nr <= 2) {
-    const int64_t elems = n * nrhs;
-    trsv::trsv_prepare_kernel<<<(unsigned)ceil_div(elems, 256), 256, 0, st>>>(n, nrhs, X, ldx,
-                                                                            B, sync);
-    LUB_LAUNCH_CHECK();
-  } else {
-    LUB_CUDA_TRY(cudaMemsetAsync(sync, 0, (size_t)(trsv::kSyncHeader + a.ngroups) * 4, st));
-  }
+  const int64_t elems = n * nrhs;
+  trsv::trsv_prepare_kernel<<<(unsigned)ceil_div(elems, 256), 256, 0, st>>>(n, nrhs, X, ldx, B,
+                                                                          sync);
+  LUB_LAUNCH_CHECK();
   const bool v16 = ((reinterpret_cast<uintptr_t>(lu) & 15) == 0) && (ld % 4 == 0);
   if (trans)
     return v16 ? trsv::launch_nr<true, true>(st, a, nr) : trsv::launch_nr<true, false>(st, a, nr);
