@@ -54,9 +54,9 @@ static TcOperand tc_kind(lu_compute c) {
 
 // Workspace for the low-precision operand copies of an M x K by K x N
 // tensor-core update: A (row-major, ld K), B (column-major, ld K), the e4m3
-// scales of both and a scratch array for the per-tile maxima.
+// scales of both.
 struct TcWs {
-  size_t off_a = 0, off_b = 0, off_sa = 0, off_sb = 0, off_tmp = 0, bytes = 0;
+  size_t off_a = 0, off_b = 0, off_sa = 0, off_sb = 0, bytes = 0;
 };
 
 static TcWs tc_ws_layout(size_t base, int64_t M, int64_t N, int64_t K,
@@ -70,7 +70,6 @@ static TcWs tc_ws_layout(size_t base, int64_t M, int64_t N, int64_t K,
   const size_t ts = (size_t)(std::max(ceil_div(M, 128), ceil_div(N, 128)) + 1) * sizeof(int);
   w.off_sa = off;  off = align_up(off + ts, 256);
   w.off_sb = off;  off = align_up(off + ts, 256);
-  w.off_tmp = off; off = align_up(off + ts, 256);
   w.bytes = off - base;
   return w;
 }
@@ -82,19 +81,14 @@ static lu_status tc_pack(cudaStream_t st, TcOperand kind, int64_t M, int64_t N,
                          int64_t K, const float* a, int64_t lda, const float* b,
                          int64_t ldb, char* ws, const TcWs& w) {
   const int64_t ldk = tc_packed_k(kind, K);
-  int* sa = nullptr;
-  int* sb = nullptr;
   ProfScope ps("pack_operands", st,
                (double)(M + N) * (4.0 * K + (double)tc_operand_bytes(kind) * ldk));
-  if (tc_scaled(kind)) {
-    sa = reinterpret_cast<int*>(ws + w.off_sa);
-    sb = reinterpret_cast<int*>(ws + w.off_sb);
-    int* tmp = reinterpret_cast<int*>(ws + w.off_tmp);
-    LUB_TRY(launch_scale_rowtiles(st, M, K, a, lda, sa, tmp, tc_scale_bound(kind)));
-    LUB_TRY(launch_scale_coltiles(st, K, N, b, ldb, sb, tmp, tc_scale_bound(kind)));
-  }
-  LUB_TRY(launch_pack_a(st, kind, M, K, a, lda, ws + w.off_a, ldk, sa));
-  LUB_TRY(launch_pack_b(st, kind, K, N, b, ldb, ws + w.off_b, ldk, sb));
+  if (tc_scaled(kind))
+    return launch_pack_scaled(st, kind, M, N, K, a, lda, ws + w.off_a,
+                              reinterpret_cast<int*>(ws + w.off_sa), b, ldb, ws + w.off_b,
+                              reinterpret_cast<int*>(ws + w.off_sb), ldk);
+  LUB_TRY(launch_pack_a(st, kind, M, K, a, lda, ws + w.off_a, ldk));
+  LUB_TRY(launch_pack_b(st, kind, K, N, b, ldb, ws + w.off_b, ldk));
   return LU_SUCCESS;
 }
 
@@ -112,22 +106,17 @@ static lu_status tc_pack_range(cudaStream_t st, TcOperand kind, int64_t r0, int6
   const int64_t es = tc_operand_bytes(kind);
   ProfScope ps("pack_operands", st,
                (double)((r1 - r0) + (c1 - c0)) * (4.0 * K + (double)es * ldk));
-  int* tmp = reinterpret_cast<int*>(ws + w.off_tmp);
-  if (r1 > r0) {
-    int* sa = scaled ? reinterpret_cast<int*>(ws + w.off_sa) + r0 / 128 : nullptr;
-    if (scaled)
-      LUB_TRY(launch_scale_rowtiles(st, r1 - r0, K, a + r0, lda, sa, tmp, tc_scale_bound(kind)));
-    LUB_TRY(launch_pack_a(st, kind, r1 - r0, K, a + r0, lda, ws + w.off_a + r0 * ldk * es,
-                          ldk, sa));
-  }
-  if (c1 > c0) {
-    int* sb = scaled ? reinterpret_cast<int*>(ws + w.off_sb) + c0 / 128 : nullptr;
-    if (scaled)
-      LUB_TRY(launch_scale_coltiles(st, K, c1 - c0, b + c0 * ldb, ldb, sb, tmp,
-                                    tc_scale_bound(kind)));
+  if (scaled)
+    return launch_pack_scaled(st, kind, r1 - r0, c1 - c0, K, a + r0, lda,
+                              ws + w.off_a + r0 * ldk * es,
+                              reinterpret_cast<int*>(ws + w.off_sa) + r0 / 128, b + c0 * ldb, ldb,
+                              ws + w.off_b + c0 * ldk * es,
+                              reinterpret_cast<int*>(ws + w.off_sb) + c0 / 128, ldk);
+  if (r1 > r0)
+    LUB_TRY(launch_pack_a(st, kind, r1 - r0, K, a + r0, lda, ws + w.off_a + r0 * ldk * es, ldk));
+  if (c1 > c0)
     LUB_TRY(launch_pack_b(st, kind, K, c1 - c0, b + c0 * ldb, ldb,
-                          ws + w.off_b + c0 * ldk * es, ldk, sb));
-  }
+                          ws + w.off_b + c0 * ldk * es, ldk));
   return LU_SUCCESS;
 }
 
@@ -631,7 +620,7 @@ static lu_status rl_factor(const Plan& p, cudaStream_t st, float* a,
     for (int b = 1; b < nbuf; ++b) {
       w2[b] = w2[0];
       w2[b].off_a += b * shift; w2[b].off_b += b * shift; w2[b].off_sa += b * shift;
-      w2[b].off_sb += b * shift; w2[b].off_tmp += b * shift;
+      w2[b].off_sb += b * shift;
     }
   }
   const bool fused = fused_pack(p.outer);
@@ -1472,9 +1461,9 @@ static lu_status ll_factor(const Plan& p, cudaStream_t st, float* a,
       // L21 rows [ofs+in, n) of the block's columns -> row-major copy;
       // U12 columns [ofs+in, n) of the block's rows -> column-major copy
       LUB_TRY(launch_pack_a(st, kind, rest, in, blk + in, lda,
-                            Lc + ((ofs + in) * ldk + ofs) * es, ldk, nullptr));
+                            Lc + ((ofs + in) * ldk + ofs) * es, ldk));
       LUB_TRY(launch_pack_b(st, kind, in, rest, blk + in * lda, lda,
-                            Uc + ((ofs + in) * ldk + ofs) * es, ldk, nullptr));
+                            Uc + ((ofs + in) * ldk + ofs) * es, ldk));
     }
   }
   LUB_CUDA_TRY(cudaEventRecord(S->ll_ready, S->update));
@@ -1935,24 +1924,40 @@ lu_status gemm_update_ex(lu_compute compute, cudaStream_t st, int64_t m, int64_t
   const int64_t ldk = tc_packed_k(TcOperand::F16, k);
   __half* ap = reinterpret_cast<__half*>(wsb + w.off_a);
   __half* bp = reinterpret_cast<__half*>(wsb + w.off_b);
-  lu_status s = launch_fill_int(st, err, 0, 1);
-  if (s == LU_SUCCESS) {
+  // fp16 B is K-major as it stands: TMA reads it in place where its base and
+  // columns are 16-byte aligned and C does not reach into it (m = 6000, n =
+  // 7000, k = 500: the copy took 18 us of 117)
+  const uintptr_t b0 = (uintptr_t)b, b1 = b0 + 2 * (uintptr_t)(ldb * (n - 1) + k);
+  const uintptr_t c0 = (uintptr_t)c;
+  const uintptr_t c1 = c0 + (tc == LU_F16 ? 2 : 4) * (uintptr_t)(ldc * (n - 1) + m);
+  const bool in_place = b0 % 16 == 0 && ldb % 8 == 0 && ldb <= INT32_MAX && (c1 <= b0 || b1 <= c0);
+  const void* bq = bp;
+  int64_t ldbq = ldk;
+  lu_status s = LU_SUCCESS;
+  {
     ProfScope ps("pack_operands", st, (double)(m + n) * (double)k * (f16ops ? 4.0 : 6.0));
     if (f16ops) {
-      s = launch_pack_a_f16(st, m, k, (const __half*)a, lda, ap, ldk);
-      if (s == LU_SUCCESS) s = launch_pack_b_f16(st, k, n, (const __half*)b, ldb, bp, ldk);
+      s = launch_pack_a_f16(st, m, k, (const __half*)a, lda, ap, ldk, err);
+      if (in_place) {
+        bq = b;
+        ldbq = ldb;
+      } else if (s == LU_SUCCESS) {
+        s = launch_pack_b_f16(st, k, n, (const __half*)b, ldb, bp, ldk);
+      }
     } else {
-      s = tc_pack(st, TcOperand::F16, m, n, k, (const float*)a, lda, (const float*)b, ldb,
-                  wsb, w);
+      s = launch_fill_int(st, err, 0, 1);
+      if (s == LU_SUCCESS)
+        s = tc_pack(st, TcOperand::F16, m, n, k, (const float*)a, lda, (const float*)b, ldb, wsb,
+                    w);
     }
   }
   if (s == LU_SUCCESS) {
     ProfScope ps("tc_update", st, (tc == LU_F32 ? 8.0 : 4.0) * m * n + 2.0 * (m + n) * k,
                  2.0 * m * n * k);
     s = tc == LU_F32 ? launch_tc_update(st, TcOperand::F16, m, n, k, (float)alpha, ap, ldk,
-                                        bp, ldk, (float*)c, ldc, nullptr, nullptr, err)
+                                        bq, ldbq, (float*)c, ldc, nullptr, nullptr, err)
                      : launch_tc_update_h(st, TcOperand::F16, m, n, k, (float)alpha, ap, ldk,
-                                          bp, ldk, (__half*)c, ldc, err);
+                                          bq, ldbq, (__half*)c, ldc, err);
   }
   if (owned) cudaFreeAsync(ws, st);
   return s;

@@ -108,30 +108,27 @@ lu_status launch_tc_update_withheld(cudaStream_t st, int64_t M, int64_t N, int64
                                     int64_t ldb_p, float* C, int64_t ldc, int* err,
                                     long long wait_cycles, int tiles_per_cta);
 
-// Largest power-of-two scale per 128-row tile of the fp32 column-major
-// src (M x K) / per 128-column tile of src (K x N) such that amax * 2^s <=
-// bound (448: e4m3 max; 32768 for split fp16).  `tmp` needs one int per tile.
-lu_status launch_scale_rowtiles(cudaStream_t st, int64_t M, int64_t K,
-                                const float* src, int64_t lds, int* scale,
-                                int* tmp, float bound = 448.0f);
-lu_status launch_scale_coltiles(cudaStream_t st, int64_t K, int64_t N,
-                                const float* src, int64_t lds, int* scale,
-                                int* tmp, float bound = 448.0f);
-
-// A operand: dst[i*ldd + k] = round(src[i + k*lds] * 2^scale[i/128])
-// (SPLIT16: the three segments, each round16(K) long, zero padded).
+// Operand copies of fp32 column-major sources, unscaled kinds (F16, BF16).
+// A: dst[i*ldd + k] = round(src[i + k*lds]).
 lu_status launch_pack_a(cudaStream_t st, TcOperand kind, int64_t M, int64_t K,
-                        const float* src, int64_t lds, void* dst, int64_t ldd,
-                        const int* scale);
-// The same copies of fp16 sources (F16 kind, no scales): A transposed into
-// the row-major copy, B into the compact column-major copy.
+                        const float* src, int64_t lds, void* dst, int64_t ldd);
+// B: dst[k + j*ldd] = round(src[k + j*lds]).
+lu_status launch_pack_b(cudaStream_t st, TcOperand kind, int64_t K, int64_t N,
+                        const float* src, int64_t lds, void* dst, int64_t ldd);
+// The same copies of fp16 sources (F16 kind): A transposed into the row-major
+// copy (clearing *err, when given, on the way), B into the compact
+// column-major copy.
 lu_status launch_pack_a_f16(cudaStream_t st, int64_t M, int64_t K, const __half* src,
-                            int64_t lds, __half* dst, int64_t ldd);
+                            int64_t lds, __half* dst, int64_t ldd, int* err = nullptr);
 lu_status launch_pack_b_f16(cudaStream_t st, int64_t K, int64_t N, const __half* src,
                             int64_t lds, __half* dst, int64_t ldd);
-// B operand: dst[k + j*ldd] = round(src[k + j*lds] * 2^scale[j/128]).
-lu_status launch_pack_b(cudaStream_t st, TcOperand kind, int64_t K, int64_t N,
-                        const float* src, int64_t lds, void* dst, int64_t ldd,
-                        const int* scale);
+// Both copies of a scaled kind in one launch (M or N may be 0): per 128-row tile
+// of A (M x K) / 128-column tile of B (K x N) the largest power-of-two scale
+// with amax * 2^s <= tc_scale_bound(kind), s to sa / sb (one int per tile), and
+// the values times 2^s (SPLIT16: the three segments, each round16(K) long, zero
+// padded), both copies with leading dimension ldd.
+lu_status launch_pack_scaled(cudaStream_t st, TcOperand kind, int64_t M, int64_t N, int64_t K,
+                             const float* a, int64_t lda, void* da, int* sa, const float* b,
+                             int64_t ldb, void* db, int* sb, int64_t ldd);
 
 }  // namespace lub
