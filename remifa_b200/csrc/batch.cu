@@ -31,10 +31,7 @@
 // multiply, fused a - l*u), the L rows below (row * 1/d, fused updates), the
 // U columns right of it (forward substitution) and a rank-8 update
 // accumulated acc = fma(l, u, acc) then subtracted (src/lu_nopiv.cu:105-326).
-// Rows are owned by threads (row p by thread p mod 256), so each 8-column
-// step costs one CTA barrier: the warp owning the tile's rows factors the
-// tile and the U strip, then every thread eliminates and updates its own
-// rows.
+// See panel_rows.cuh.
 #include "common.cuh"
 #include "kernels.cuh"
 #include "panel_rows.cuh"
@@ -76,7 +73,7 @@ struct Misc {
   int item;
   int bad;
   int abort;
-  float inv[2][8];
+  float inv[8];
 };
 
 struct BatchArgs {
@@ -541,7 +538,7 @@ __global__ void __launch_bounds__(kT, 1) batch_lu_kernel(BatchArgs a) {
         if (ms->abort) break;
       }
       if (ms->abort) break;
-      rows::panel_block<kT>(C, ldc, n, c0, wj, &ms->inv[0][0], &ms->bad, c0);
+      rows::panel_block<kT>(C, ldc, n, c0, wj, ms->inv, &ms->bad, c0);
       store_block(A + (int64_t)c0 * lda, lda, n, wj, vec, C, ldc);
       // the later block columns' outer updates read this one's L rows as
       // fp16 operand images, by bulk copy
