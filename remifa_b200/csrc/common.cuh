@@ -156,6 +156,35 @@ __device__ __forceinline__ bool factor_tile8_fast(float* T, int LD, float* inv) 
   return true;
 }
 
+// Programmatic dependent launch: a kernel launched with launch_dependent may be
+// placed on the SMs while the kernel before it in the stream still runs, and
+// waits (before it reads or writes anything) until that one has completed and
+// its results are visible.  dependents_launch lets the next one be placed, from
+// the moment all CTAs have called it (or exited); a kernel that never calls it
+// still hides its successor's launch.  Kernels that take tensor memory take it
+// after dependency_wait and call dependents_launch after that: one that waits
+// holds none.  A factorization's critical path is 4 or 5 small kernels per 128
+// columns: n = 200 67.5 -> 56.4 us, 2000 (with its solves) 1180 -> 1093, fp16
+// operands at 5001 1966 -> 1870, e4m3 at 8192 4570 -> 4224.
+__device__ __forceinline__ void dependency_wait() { cudaGridDependencySynchronize(); }
+__device__ __forceinline__ void dependents_launch() { cudaTriggerProgrammaticLaunchCompletion(); }
+
+template <typename... P, typename... A>
+inline cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
+                                    cudaStream_t st, A&&... args) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // Record the 1-based global index of a zero / non-finite pivot.
 __device__ __forceinline__ void note_pivot(float d, int64_t col0,
                                            int* first_bad) {

@@ -11,6 +11,8 @@ namespace lub {
 namespace {
 
 __global__ void fill_int_kernel(int* p, int v, int64_t count) {
+  dependency_wait();
+  dependents_launch();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < count) p[i] = v;
 }
@@ -19,6 +21,7 @@ __global__ void fill_int_kernel(int* p, int v, int64_t count) {
 // -1 if a bounded device-side wait gave up (err non-zero).
 __global__ void finalize_info_kernel(const int* first_bad, const int* err,
                                      int* info) {
+  dependency_wait();
   const int f = *first_bad;
   *info = (err != nullptr && *err != 0) ? -1 : (f == kNoBadPivot) ? 0 : f;
 }
@@ -79,14 +82,14 @@ cudaError_t set_smem_limit(const void* func, size_t bytes) {
 
 lu_status launch_fill_int(cudaStream_t st, int* p, int v, int64_t count) {
   if (count <= 0) return LU_SUCCESS;
-  fill_int_kernel<<<(unsigned)ceil_div(count, 256), 256, 0, st>>>(p, v, count);
+  LUB_CUDA_TRY(launch_dependent(fill_int_kernel, (unsigned)ceil_div(count, 256), 256, 0, st, p, v, count));
   LUB_LAUNCH_CHECK();
   return LU_SUCCESS;
 }
 
 lu_status launch_finalize_info(cudaStream_t st, const int* first_bad,
                                const int* err, int* info) {
-  finalize_info_kernel<<<1, 1, 0, st>>>(first_bad, err, info);
+  LUB_CUDA_TRY(launch_dependent(finalize_info_kernel, 1, 1, 0, st, first_bad, err, info));
   LUB_LAUNCH_CHECK();
   return LU_SUCCESS;
 }
