@@ -113,8 +113,8 @@ lu_status refine_multi(lu_stream_t stream, int64_t n, int64_t nrhs, const float*
                 : launch_norm_inf(st, n, d_a, lda, P, mnorm));
   LUB_CUDA_TRY(cudaMemcpy2DAsync(d_x, (size_t)ldx * 8, d_b, (size_t)ldb * 8, (size_t)n * 8,
                                  (size_t)nrhs, cudaMemcpyDeviceToDevice, st));
-  // the solves copy their right-hand sides into R (free until the next
-  // residual) and count tickets in the sync words
+  // the solves pass through R or D (free until the next residual) and count
+  // tickets in the sync words
   unsigned* sync = reinterpret_cast<unsigned*>(wb + w.off_sync);
   LUB_TRY(launch_lu_solve(st, n, d_lu, ldlu, d_x, ldx, nrhs, trans != 0, sync, R));
   for (;;) {
@@ -142,9 +142,8 @@ lu_status refine_multi(lu_stream_t stream, int64_t n, int64_t nrhs, const float*
       e = std::max(e, ec);
     }
     if (std::isnan(e) || e <= tol || it >= max_iter) break;
-    LUB_CUDA_TRY(cudaMemcpyAsync(D, R, (size_t)n * nrhs * 8, cudaMemcpyDeviceToDevice, st));
-    LUB_TRY(launch_lu_solve(st, n, d_lu, ldlu, D, n, nrhs, trans != 0, sync, R));
-    LUB_TRY(launch_axpy(st, n, nrhs, D, d_x, ldx));
+    LUB_TRY(launch_lu_solve(st, n, d_lu, ldlu, R, n, nrhs, trans != 0, sync, D));
+    LUB_TRY(launch_axpy(st, n, nrhs, R, d_x, ldx));
     ++it;
   }
   if (iters) *iters = it;

@@ -49,9 +49,13 @@ constexpr unsigned long long kWaitNs = 4000000000ull;  // bound of one wait
 struct Args {
   const float* lu;
   int64_t ld;
-  double* X;        // solutions, written in place
+  double* X;        // solutions, all pending at the start
   int64_t ldx;
-  const double* B;  // right-hand sides (n x nrhs, ld n)
+  double* B;        // right-hand sides
+  int64_t ldb;
+  int mark;         // leave B pending: the next pass publishes its solution there
+  int early;        // LU and the sync words are ready before the kernel in front
+                    // of this one ends: only B and X wait for it
   int64_t n;
   int64_t nrhs;
   int nblk;
@@ -533,6 +537,8 @@ trsv_kernel(Args a) {
   int* ctrl = reinterpret_cast<int*>(xin + kCluster * NR * BS);
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (!a.early) dependency_wait();
+  dependents_launch();
   // the cluster's ticket: its kCluster consecutive row blocks of one group
   const int rank = cluster_rank();
   for (int e = tid; e < kCluster * NR * BS; e += kThreads)
@@ -588,21 +594,30 @@ trsv_kernel(Args a) {
 #pragma unroll
   for (int q = 0; q < S - 1; ++q) issue(q);
   double xq[PD][NX][NR];
+  double bm[2][NR];   // right-hand sides of rows lane and lane + 32
+  auto fetch_inputs = [&]() {
 #pragma unroll
-  for (int d = 0; d < PD; ++d)
-    if (d < nglob) fetch_x<NX, NR>(xq[d], a, tile_k0(d), tile_kw(d), c0, nc, kb, ks);
-  // right-hand sides of rows lane and lane + 32
-  double bm[2][NR];
+    for (int d = 0; d < PD; ++d)
+      if (d < nglob) fetch_x<NX, NR>(xq[d], a, tile_k0(d), tile_kw(d), c0, nc, kb, ks);
 #pragma unroll
-  for (int h = 0; h < 2; ++h)
+    for (int h = 0; h < 2; ++h)
 #pragma unroll
-    for (int c = 0; c < NR; ++c) {
-      const int r = lane + 32 * h;
-      bm[h][c] = (r < rw && c < nc) ? a.B[(r0 + r) + (c0 + c) * a.n] : 0.0;
-    }
+      for (int c = 0; c < NR; ++c) {
+        const int r = lane + 32 * h;
+        bm[h][c] = (r < rw && c < nc) ? a.B[(r0 + r) + (c0 + c) * a.ldb] : 0.0;
+      }
+  };
+  if (!a.early) fetch_inputs();
 
   cp_wait<S - 1>();
   __syncthreads();
+  if (a.mark && warp == 0)   // every warp has its copy
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int c = 0; c < NR; ++c)
+        if (lane + 32 * h < rw && c < nc)
+          a.B[(r0 + lane + 32 * h) + (c0 + c) * a.ldb] = __longlong_as_double((long long)kPending);
   invert_diag<TRANS>(Dsrc, Dinv, rdiag, rw, fwd, a.unit != 0);
 
   // ---- W = Dinv * op(T)[block, previous block] ----
@@ -633,6 +648,11 @@ trsv_kernel(Args a) {
           W[i][1] = fma(d, (double)tk[1][mm], W[i][1]);
         }
     }
+  }
+
+  if (a.early) {
+    dependency_wait();
+    fetch_inputs();
   }
 
   // ---- bulk: the tiles before the previous block's, per warp.
@@ -776,18 +796,24 @@ trsv_kernel(Args a) {
 
 // B <- X and X <- pending, for the rows and columns of the solve; the first
 // thread also clears the ticket counter and the expired-wait count.
+constexpr int kHeader = 4;   // words of a pass's sync area: ticket, expired waits, spare
+
+// Clears the ticket and expiry words of both passes' sync areas and marks the
+// n x nrhs solutions at Y (dense) pending; X given: moves X there first and
+// marks X itself (one pass in place).
 __global__ void trsv_prepare_kernel(int64_t n, int64_t nrhs, double* __restrict__ X,
-                                    int64_t ldx, double* __restrict__ B,
+                                    int64_t ldx, double* __restrict__ Y,
                                     unsigned* __restrict__ sync) {
+  dependency_wait();
   const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e == 0) {
-    sync[0] = 0;
-    sync[1] = 0;
-  }
+  if (e == 0) sync[0] = sync[1] = sync[kHeader] = sync[kHeader + 1] = 0;
   if (e >= n * nrhs) return;
-  const int64_t c = e / n, i = e - c * n;
-  double* p = X + i + c * ldx;
-  B[e] = *p;
+  double* p = Y + e;
+  if (X) {
+    const int64_t c = e / n, i = e - c * n;
+    p = X + i + c * ldx;
+    Y[e] = *p;
+  }
   *p = __longlong_as_double((long long)kPending);
 }
 
@@ -804,7 +830,6 @@ __global__ void trsv_prepare_kernel(int64_t n, int64_t nrhs, double* __restrict_
 
 constexpr int DS = BS + 4;   // row stride of Dinv: conflict-free fragment reads
 constexpr int YS = 12;       // row stride of y, likewise
-constexpr int kHeader = 4;   // words of the sync area: ticket, expired waits, spare
 
 constexpr size_t mma_smem_bytes() {
   return (size_t)BS * DS * 8          // inverse of the diagonal block (fp64)
@@ -829,6 +854,8 @@ trsv_mma_kernel(Args a) {
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int lr = lane >> 2, lk = lane & 3;
+  if (!a.early) dependency_wait();
+  dependents_launch();
   if (tid == 0) ctrl[0] = (int)atomicAdd(a.sync, 1u);
   __syncthreads();
   const int ticket = ctrl[0];
@@ -882,17 +909,25 @@ trsv_mma_kernel(Args a) {
   };
   float cur[8][2], nxt[8][2];
   double xq[PD][2];
-#pragma unroll
-  for (int d = 0; d < PD; ++d)
-    if (d < nbulk) fetch(xq[d], d);
-  if (nbulk > 0) load_a(0, cur);
   // right-hand side entries (row tid / 4, columns 2 (tid & 3) and the next)
   double bm[2];
+  auto fetch_inputs = [&]() {
 #pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const int r = tid >> 2, c = 2 * (tid & 3) + h;
-    bm[h] = (r < rw && c < nc) ? a.B[(r0 + r) + (c0 + c) * a.n] : 0.0;
-  }
+    for (int d = 0; d < PD; ++d)
+      if (d < nbulk) fetch(xq[d], d);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int r = tid >> 2, c = 2 * (tid & 3) + h;
+      double* p = a.B + (r0 + r) + (c0 + c) * a.ldb;
+      bm[h] = 0.0;
+      if (r < rw && c < nc) {
+        bm[h] = *p;
+        if (a.mark) *p = __longlong_as_double((long long)kPending);
+      }
+    }
+  };
+  if (!a.early) fetch_inputs();
+  if (nbulk > 0) load_a(0, cur);
   cp_wait<0>();
   __syncthreads();
   invert_diag<TRANS, DS>(Dsrc, Dinv, rdiag, rw, fwd, a.unit != 0);
@@ -910,6 +945,11 @@ trsv_mma_kernel(Args a) {
 #pragma unroll
       for (int f = 0; f < 8; ++f) mma64(W[f], d, (double)Tw[tile_index<TRANS>(k, 8 * f + lr)]);
     }
+  }
+
+  if (a.early) {
+    dependency_wait();
+    fetch_inputs();
   }
 
   // ---- bulk: the tiles before the previous block's
@@ -1019,18 +1059,21 @@ lu_status launch_one(cudaStream_t st, const Args& a) {
     cfg.blockDim = dim3(kThreads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute at[1];
+    cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = kCluster;
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = 2;
     LUB_CUDA_TRY(cudaLaunchKernelEx(&cfg, fn, a));
   } else {
     smem = mma_smem_bytes();
     fn = trsv_mma_kernel<TRANS, V16>;
     LUB_CUDA_TRY(set_smem_limit((const void*)fn, smem));
-    fn<<<(unsigned)((int64_t)a.nblk * a.ngroups), kThreads, smem, st>>>(a);
+    LUB_CUDA_TRY(launch_dependent(fn, (unsigned)((int64_t)a.nblk * a.ngroups), kThreads, smem, st,
+                                  a));
   }
   LUB_LAUNCH_CHECK();
   return LU_SUCCESS;
@@ -1061,6 +1104,8 @@ __global__ void __launch_bounds__(kT)
 residual_partial_kernel(int64_t n, const float* __restrict__ A, int64_t lda,
                         const double* __restrict__ x, double* __restrict__ P) {
   __shared__ double xs[kRC];
+  dependency_wait();
+  dependents_launch();
   const int64_t c0 = (int64_t)blockIdx.y * kRC;
   const int cn = (int)((n - c0) < kRC ? (n - c0) : kRC);
   for (int k = threadIdx.x; k < cn; k += kT) xs[k] = x[c0 + k];
@@ -1069,7 +1114,8 @@ residual_partial_kernel(int64_t n, const float* __restrict__ A, int64_t lda,
   if (i >= n) return;
   const float* col = A + i + c0 * lda;
   double acc = 0.0;
-#pragma unroll 8
+  // few CTAs at the sizes a single solve has: 32 loads in flight per thread
+#pragma unroll 32
   for (int k = 0; k < cn; ++k) acc = fma((double)col[k * lda], xs[k], acc);
   P[(int64_t)blockIdx.y * n + i] = acc;
 }
@@ -1081,6 +1127,7 @@ __global__ void __launch_bounds__(kT)
 residual_final_kernel(int64_t n, int nchunks, const double* __restrict__ P,
                       const double* __restrict__ b, const double* __restrict__ x,
                       double* __restrict__ r, unsigned long long* __restrict__ maxes) {
+  dependency_wait();
   const int64_t i = (int64_t)blockIdx.x * kT + threadIdx.x;
   double ri = 0.0, xi = 0.0, bi = 0.0;
   if (i < n) {
@@ -1111,6 +1158,7 @@ rowsum_partial_kernel(int64_t n, const float* __restrict__ A, int64_t lda,
   if (i >= n) return;
   const float* col = A + i + c0 * lda;
   double acc = 0.0;
+#pragma unroll 32
   for (int k = 0; k < cn; ++k) acc += fabs((double)col[k * lda]);
   P[(int64_t)blockIdx.y * n + i] = acc;
 }
@@ -1129,6 +1177,8 @@ rowsum_final_kernel(int64_t n, int nchunks, const double* __restrict__ P,
 // X += D (n x nrhs, D dense): one launch for all columns.
 __global__ void axpy_kernel(int64_t n, int64_t nrhs, const double* __restrict__ d,
                             double* __restrict__ x, int64_t ldx) {
+  dependency_wait();
+  dependents_launch();
   const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (e < n * nrhs) {
     const int64_t c = e / n;
@@ -1341,7 +1391,7 @@ lu_status launch_residual_nf(cudaStream_t st, int64_t n, int64_t nrhs, const flo
 
 size_t trsm_sync_bytes(int64_t nrhs) {
   (void)nrhs;
-  return align_up((size_t)trsv::kHeader * 4, 256);
+  return align_up((size_t)2 * trsv::kHeader * 4, 256);
 }
 
 size_t trsm_ws_bytes(int64_t n, int64_t nrhs) {
@@ -1349,12 +1399,12 @@ size_t trsm_ws_bytes(int64_t n, int64_t nrhs) {
          align_up((size_t)(n < 0 ? 0 : n) * (size_t)(nrhs < 0 ? 0 : nrhs) * 8, 256);
 }
 
-lu_status launch_trsm(cudaStream_t st, int64_t n, const float* lu, int64_t ld,
-                      double* X, int64_t ldx, int64_t nrhs, bool upper,
-                      bool trans, unsigned* sync, double* B,
-                      unsigned long long wait_ns, int withhold) {
-  if (n <= 0 || nrhs <= 0) return LU_SUCCESS;
-  if (!sync || !B) return LU_ERR_INVALID_ARG;
+namespace {
+// One pass: op(T) X = B.
+lu_status launch_pass(cudaStream_t st, int64_t n, const float* lu, int64_t ld, double* X,
+                      int64_t ldx, double* B, int64_t ldb, int64_t nrhs, bool upper, bool trans,
+                      unsigned* sync, bool mark, bool early, unsigned long long wait_ns,
+                      int withhold) {
   const int nr = trsv::group_width(nrhs);
   if (ceil_div(n, trsv::BS) * ceil_div(nrhs, nr) > 0x7fffffffll) return LU_ERR_INVALID_ARG;
   trsv::Args a;
@@ -1363,6 +1413,9 @@ lu_status launch_trsm(cudaStream_t st, int64_t n, const float* lu, int64_t ld,
   a.X = X;
   a.ldx = ldx;
   a.B = B;
+  a.ldb = ldb;
+  a.mark = mark;
+  a.early = early;
   a.n = n;
   a.nrhs = nrhs;
   a.nblk = (int)ceil_div(n, trsv::BS);
@@ -1373,26 +1426,50 @@ lu_status launch_trsm(cudaStream_t st, int64_t n, const float* lu, int64_t ld,
   a.sync = sync;
   a.wait_ns = wait_ns > 0 ? wait_ns : trsv::kWaitNs;
   a.withhold = withhold;
-  const int64_t elems = n * nrhs;
-  trsv::trsv_prepare_kernel<<<(unsigned)ceil_div(elems, 256), 256, 0, st>>>(n, nrhs, X, ldx, B,
-                                                                          sync);
-  LUB_LAUNCH_CHECK();
   const bool v16 = ((reinterpret_cast<uintptr_t>(lu) & 15) == 0) && (ld % 4 == 0);
   if (trans)
     return v16 ? trsv::launch_nr<true, true>(st, a, nr) : trsv::launch_nr<true, false>(st, a, nr);
   return v16 ? trsv::launch_nr<false, true>(st, a, nr) : trsv::launch_nr<false, false>(st, a, nr);
 }
 
+lu_status launch_prepare(cudaStream_t st, int64_t n, int64_t nrhs, double* X, int64_t ldx,
+                         double* Y, unsigned* sync) {
+  const int64_t blocks = ceil_div(n * nrhs, 256);
+  LUB_CUDA_TRY(launch_dependent(trsv::trsv_prepare_kernel, (unsigned)blocks, 256, 0, st, n, nrhs,
+                                X, ldx, Y, sync));
+  LUB_LAUNCH_CHECK();
+  return LU_SUCCESS;
+}
+}  // namespace
+
+lu_status launch_trsm(cudaStream_t st, int64_t n, const float* lu, int64_t ld,
+                      double* X, int64_t ldx, int64_t nrhs, bool upper,
+                      bool trans, unsigned* sync, double* B,
+                      unsigned long long wait_ns, int withhold) {
+  if (n <= 0 || nrhs <= 0) return LU_SUCCESS;
+  if (!sync || !B) return LU_ERR_INVALID_ARG;
+  LUB_TRY(launch_prepare(st, n, nrhs, X, ldx, B, sync));
+  return launch_pass(st, n, lu, ld, X, ldx, B, n, nrhs, upper, trans, sync, false, false, wait_ns,
+                     withhold);
+}
+
+// The first pass takes its right-hand sides from X, leaves X pending and solves
+// into Y; the second solves from Y into X.  So one preparing launch serves both,
+// and the second pass may be placed while the first still runs: its set-up (the
+// inverse of the diagonal block and its product with the neighbouring tile, ~14
+// us) reads only the factors, which were complete before the first pass began
+// (n = 10007: 297 -> 277.5 us; a preparing launch and a set-up per pass before).
 lu_status launch_lu_solve(cudaStream_t st, int64_t n, const float* lu, int64_t ld,
                           double* X, int64_t ldx, int64_t nrhs, bool trans, unsigned* sync,
-                          double* B) {
-  if (!trans) {  // L U x = b: L y = b, then U x = y
-    LUB_TRY(launch_trsm(st, n, lu, ld, X, ldx, nrhs, false, false, sync, B));
-    return launch_trsm(st, n, lu, ld, X, ldx, nrhs, true, false, sync, B);
-  }
-  // (L U)^T x = U^T L^T x = b: U^T y = b, then L^T x = y
-  LUB_TRY(launch_trsm(st, n, lu, ld, X, ldx, nrhs, true, true, sync, B));
-  return launch_trsm(st, n, lu, ld, X, ldx, nrhs, false, true, sync, B);
+                          double* Y) {
+  if (n <= 0 || nrhs <= 0) return LU_SUCCESS;
+  if (!sync || !Y) return LU_ERR_INVALID_ARG;
+  LUB_TRY(launch_prepare(st, n, nrhs, nullptr, 0, Y, sync));
+  // L U x = b: L y = b, then U x = y; (L U)^T x = U^T L^T x = b: U^T y = b, then
+  // L^T x = y
+  LUB_TRY(launch_pass(st, n, lu, ld, Y, n, X, ldx, nrhs, trans, trans, sync, true, false, 0, -1));
+  return launch_pass(st, n, lu, ld, X, ldx, Y, n, nrhs, !trans, trans, sync + trsv::kHeader, false,
+                     true, 0, -1);
 }
 
 size_t residual_ws_bytes(int64_t n) {
@@ -1406,9 +1483,10 @@ lu_status launch_residual(cudaStream_t st, int64_t n, const float* A,
   double* P = static_cast<double*>(ws);
   LUB_CUDA_TRY(cudaMemsetAsync(maxes, 0, 3 * sizeof(unsigned long long), st));
   dim3 g((unsigned)ceil_div(n, kT), (unsigned)nch);
-  residual_partial_kernel<<<g, kT, 0, st>>>(n, A, lda, x, P);
+  LUB_CUDA_TRY(launch_dependent(residual_partial_kernel, g, kT, 0, st, n, A, lda, x, P));
   LUB_LAUNCH_CHECK();
-  residual_final_kernel<<<(unsigned)ceil_div(n, kT), kT, 0, st>>>(n, nch, P, b, x, r, maxes);
+  LUB_CUDA_TRY(launch_dependent(residual_final_kernel, (unsigned)ceil_div(n, kT), kT, 0, st, n, nch,
+                                P, b, x, r, maxes));
   LUB_LAUNCH_CHECK();
   return LU_SUCCESS;
 }
@@ -1439,7 +1517,8 @@ lu_status launch_residual_multi(cudaStream_t st, int64_t n, int64_t nrhs, const 
 lu_status launch_axpy(cudaStream_t st, int64_t n, int64_t nrhs, const double* d, double* x,
                       int64_t ldx) {
   if (n <= 0 || nrhs <= 0) return LU_SUCCESS;
-  axpy_kernel<<<(unsigned)ceil_div(n * nrhs, 256), 256, 0, st>>>(n, nrhs, d, x, ldx);
+  LUB_CUDA_TRY(launch_dependent(axpy_kernel, (unsigned)ceil_div(n * nrhs, 256), 256, 0, st, n, nrhs,
+                                d, x, ldx));
   LUB_LAUNCH_CHECK();
   return LU_SUCCESS;
 }
