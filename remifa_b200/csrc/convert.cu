@@ -60,7 +60,6 @@ __global__ void __launch_bounds__(kThreads)
 convert_kernel(int64_t m, int64_t n, const TI* __restrict__ a, int64_t lda,
                TO* __restrict__ out, int64_t ldo, int s) {
   dependency_wait();
-  dependents_launch();
   const int64_t i0 = ((int64_t)blockIdx.x * kThreads + threadIdx.x) * kVec;
   if (i0 >= m) return;
   for (int64_t j = blockIdx.y; j < n; j += gridDim.y) {
@@ -118,9 +117,11 @@ lu_status launch_typed(cudaStream_t st, int64_t m, int64_t n, const void* a,
   dim3 grid((unsigned)ceil_div(m, kRowsPerBlock),
             (unsigned)std::min<int64_t>(n, 65535));
   if (vec)
-    LUB_CUDA_TRY(launch_dependent(convert_kernel<TI, TO, true>, grid, kThreads, 0, st, m, n, (const TI*)a, lda, (TO*)out, ldo, s));
+    LUB_CUDA_TRY(launch_dependent(convert_kernel<TI, TO, true>, grid, kThreads, 0, st, m, n,
+                                  (const TI*)a, lda, (TO*)out, ldo, s));
   else
-    LUB_CUDA_TRY(launch_dependent(convert_kernel<TI, TO, false>, grid, kThreads, 0, st, m, n, (const TI*)a, lda, (TO*)out, ldo, s));
+    LUB_CUDA_TRY(launch_dependent(convert_kernel<TI, TO, false>, grid, kThreads, 0, st, m, n,
+                                  (const TI*)a, lda, (TO*)out, ldo, s));
   LUB_LAUNCH_CHECK();
   return LU_SUCCESS;
 }

@@ -32,7 +32,6 @@ sgemm_update_kernel(int64_t M, int64_t N, int64_t K, float alpha,
   __shared__ __align__(16) float As[2][BK][BM];
   __shared__ __align__(16) float Bs[2][BK][BN];
   dependency_wait();
-  dependents_launch();
 
   const int tid = threadIdx.x;
   const int tx = tid % 16, ty = tid / 16;
@@ -178,7 +177,6 @@ sgemm_update64_kernel(int64_t M, int64_t N, int64_t K, float alpha,
   __shared__ __align__(16) float As[2][BK][TB];
   __shared__ __align__(16) float Bs[2][BK][TB];
   dependency_wait();
-  dependents_launch();
   const int tid = threadIdx.x;
   const int tx = tid % 16, ty = tid / 16;
   const int64_t m0 = (int64_t)blockIdx.x * TB;
@@ -292,7 +290,6 @@ sgemm_chunk8_kernel(ChunkRegion r0, ChunkRegion r1) {
   constexpr int CB = 16 * TM;            // tile edge
   constexpr int LB = CB + 4;             // row length of the B panel
   dependency_wait();
-  dependents_launch();
   extern __shared__ __align__(16) float smem[];
   float* As = smem;                      // [Kp][CB]: As[k*CB + m]
   float* Bs = smem + kChunkMaxK * CB;    // [Kp][LB]: Bs[k*LB + n]
@@ -445,22 +442,28 @@ lu_status launch_sgemm_update(cudaStream_t st, int64_t M, int64_t N, int64_t K,
     const bool v2 = (lda % 2 == 0) && (ldb % 2 == 0) && ((uintptr_t)A % 8 == 0) &&
                     ((uintptr_t)B % 8 == 0);
     if (v2)
-      LUB_CUDA_TRY(launch_dependent(sgemm_update64_kernel<true>, g64, NT, 0, st, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc));
+      LUB_CUDA_TRY(launch_dependent(sgemm_update64_kernel<true>, g64, NT, 0, st, M, N, K, alpha,
+                                    A, lda, B, ldb, beta, C, ldc));
     else
-      LUB_CUDA_TRY(launch_dependent(sgemm_update64_kernel<false>, g64, NT, 0, st, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc));
+      LUB_CUDA_TRY(launch_dependent(sgemm_update64_kernel<false>, g64, NT, 0, st, M, N, K, alpha,
+                                    A, lda, B, ldb, beta, C, ldc));
     LUB_LAUNCH_CHECK();
     return LU_SUCCESS;
   }
   if (chunk8) {
     if (vec)
-      LUB_CUDA_TRY(launch_dependent(sgemm_update_kernel<true, true>, grid, NT, 0, st, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc));
+      LUB_CUDA_TRY(launch_dependent(sgemm_update_kernel<true, true>, grid, NT, 0, st, M, N, K,
+                                    alpha, A, lda, B, ldb, beta, C, ldc));
     else
-      LUB_CUDA_TRY(launch_dependent(sgemm_update_kernel<true, false>, grid, NT, 0, st, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc));
+      LUB_CUDA_TRY(launch_dependent(sgemm_update_kernel<true, false>, grid, NT, 0, st, M, N, K,
+                                    alpha, A, lda, B, ldb, beta, C, ldc));
   } else {
     if (vec)
-      LUB_CUDA_TRY(launch_dependent(sgemm_update_kernel<false, true>, grid, NT, 0, st, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc));
+      LUB_CUDA_TRY(launch_dependent(sgemm_update_kernel<false, true>, grid, NT, 0, st, M, N, K,
+                                    alpha, A, lda, B, ldb, beta, C, ldc));
     else
-      LUB_CUDA_TRY(launch_dependent(sgemm_update_kernel<false, false>, grid, NT, 0, st, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc));
+      LUB_CUDA_TRY(launch_dependent(sgemm_update_kernel<false, false>, grid, NT, 0, st, M, N, K,
+                                    alpha, A, lda, B, ldb, beta, C, ldc));
   }
   LUB_LAUNCH_CHECK();
   return LU_SUCCESS;

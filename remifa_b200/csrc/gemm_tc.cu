@@ -179,7 +179,6 @@ tc_update_kernel(const __grid_constant__ TcMaps maps,
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  dependents_launch();  // tensor memory is held: dependents take theirs after us
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0) {
@@ -557,7 +556,6 @@ tc_update_pair_kernel(const __grid_constant__ TcMaps maps,
   tc_fence_before();
   cluster_sync();  // both CTAs' barriers initialised and tensor memory allocated
   tc_fence_after();
-  dependents_launch();
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0) {
@@ -905,32 +903,40 @@ lu_status tc_update_impl(cudaStream_t st, TcOperand kind, int64_t M, int64_t N,
   if (part) {
     if (kind != TcOperand::F16 && kind != TcOperand::BF16) return LU_ERR_UNSUPPORTED;
     LUB_CUDA_TRY(set_smem_limit((const void*)tc_update_kernel<0, 4>, smem_bytes<4>()));
-    LUB_CUDA_TRY(launch_dependent(tc_update_kernel<0, 4>, grid, kThreads, smem_bytes<4>(), st, maps, mc, p, idesc));
+    LUB_CUDA_TRY(launch_dependent(tc_update_kernel<0, 4>, grid, kThreads, smem_bytes<4>(), st,
+                                  maps, mc, p, idesc));
   } else if (c_half) {
     if (kind != TcOperand::F16 && kind != TcOperand::BF16) return LU_ERR_UNSUPPORTED;
     LUB_CUDA_TRY(set_smem_limit((const void*)tc_update_kernel<0, 2>, smem_bytes<2>()));
-    LUB_CUDA_TRY(launch_dependent(tc_update_kernel<0, 2>, grid, kThreads, smem_bytes<2>(), st, maps, mc, p, idesc));
+    LUB_CUDA_TRY(launch_dependent(tc_update_kernel<0, 2>, grid, kThreads, smem_bytes<2>(), st,
+                                  maps, mc, p, idesc));
   } else if (kind == TcOperand::E4M3) {
     if (tma_c && !stream_c) {
       LUB_CUDA_TRY(set_smem_limit((const void*)tc_update_kernel<1, 1>, smem_bytes<1>()));
-      LUB_CUDA_TRY(launch_dependent(tc_update_kernel<1, 1>, grid, kThreads, smem_bytes<1>(), st, maps, mc, p, idesc));
+      LUB_CUDA_TRY(launch_dependent(tc_update_kernel<1, 1>, grid, kThreads, smem_bytes<1>(), st,
+                                    maps, mc, p, idesc));
     } else if (tma_c) {
       LUB_CUDA_TRY(set_smem_limit((const void*)tc_update_kernel<1, 3>, smem_bytes<3>()));
-      LUB_CUDA_TRY(launch_dependent(tc_update_kernel<1, 3>, grid, kThreads, smem_bytes<3>(), st, maps, mc, p, idesc));
+      LUB_CUDA_TRY(launch_dependent(tc_update_kernel<1, 3>, grid, kThreads, smem_bytes<3>(), st,
+                                    maps, mc, p, idesc));
     } else {
       LUB_CUDA_TRY(set_smem_limit((const void*)tc_update_kernel<1, 0>, smem_bytes<0>()));
-      LUB_CUDA_TRY(launch_dependent(tc_update_kernel<1, 0>, grid, kThreads, smem_bytes<0>(), st, maps, mc, p, idesc));
+      LUB_CUDA_TRY(launch_dependent(tc_update_kernel<1, 0>, grid, kThreads, smem_bytes<0>(), st,
+                                    maps, mc, p, idesc));
     }
   } else {
     if (tma_c && !stream_c) {
       LUB_CUDA_TRY(set_smem_limit((const void*)tc_update_kernel<0, 1>, smem_bytes<1>()));
-      LUB_CUDA_TRY(launch_dependent(tc_update_kernel<0, 1>, grid, kThreads, smem_bytes<1>(), st, maps, mc, p, idesc));
+      LUB_CUDA_TRY(launch_dependent(tc_update_kernel<0, 1>, grid, kThreads, smem_bytes<1>(), st,
+                                    maps, mc, p, idesc));
     } else if (tma_c) {
       LUB_CUDA_TRY(set_smem_limit((const void*)tc_update_kernel<0, 3>, smem_bytes<3>()));
-      LUB_CUDA_TRY(launch_dependent(tc_update_kernel<0, 3>, grid, kThreads, smem_bytes<3>(), st, maps, mc, p, idesc));
+      LUB_CUDA_TRY(launch_dependent(tc_update_kernel<0, 3>, grid, kThreads, smem_bytes<3>(), st,
+                                    maps, mc, p, idesc));
     } else {
       LUB_CUDA_TRY(set_smem_limit((const void*)tc_update_kernel<0, 0>, smem_bytes<0>()));
-      LUB_CUDA_TRY(launch_dependent(tc_update_kernel<0, 0>, grid, kThreads, smem_bytes<0>(), st, maps, mc, p, idesc));
+      LUB_CUDA_TRY(launch_dependent(tc_update_kernel<0, 0>, grid, kThreads, smem_bytes<0>(), st,
+                                    maps, mc, p, idesc));
     }
   }
   LUB_LAUNCH_CHECK();
@@ -1016,7 +1022,8 @@ lu_status tc_update_pair_impl(cudaStream_t st, TcOperand kind, int64_t M, int64_
       std::max(1, std::min({tiles, (max_ctas > 0 ? max_ctas : sm_count()) / 2, resident}));
   const uint32_t f = kind == TcOperand::BF16 ? 1u : 0u;
   const uint32_t idesc = sm100::make_idesc(f, f, 2 * kPairRows, BN);
-  LUB_CUDA_TRY(launch_dependent(tc_update_pair_kernel, 2 * pairs, kThreads, pair_smem_bytes(), st, maps, mc, p, idesc));
+  LUB_CUDA_TRY(launch_dependent(tc_update_pair_kernel, 2 * pairs, kThreads, pair_smem_bytes(), st,
+                                maps, mc, p, idesc));
   LUB_LAUNCH_CHECK();
   return LU_SUCCESS;
 }
@@ -1078,7 +1085,6 @@ splitk_finish_kernel(int64_t M, int S, const float* __restrict__ part, int64_t p
                      int64_t part_stride, float alpha, CT* __restrict__ C, int64_t ldc,
                      float* __restrict__ shadow, int64_t lds) {
   dependency_wait();
-  dependents_launch();
   const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
   const int64_t j = blockIdx.y;
   if (i >= M) return;
@@ -1131,9 +1137,11 @@ lu_status launch_splitk_finish(cudaStream_t st, int64_t M, int64_t N, int S, con
   const int64_t pld = (M + 3) / 4 * 4;
   dim3 grid((unsigned)ceil_div(M, 256), (unsigned)N);
   if (c_half)
-    LUB_CUDA_TRY(launch_dependent(splitk_finish_kernel<__half>, grid, 256, 0, st, M, S, part, pld, pld * N, alpha, static_cast<__half*>(C), ldc, shadow, lds));
+    LUB_CUDA_TRY(launch_dependent(splitk_finish_kernel<__half>, grid, 256, 0, st, M, S, part, pld,
+                                  pld * N, alpha, static_cast<__half*>(C), ldc, shadow, lds));
   else
-    LUB_CUDA_TRY(launch_dependent(splitk_finish_kernel<float>, grid, 256, 0, st, M, S, part, pld, pld * N, alpha, static_cast<float*>(C), ldc, shadow, lds));
+    LUB_CUDA_TRY(launch_dependent(splitk_finish_kernel<float>, grid, 256, 0, st, M, S, part, pld,
+                                  pld * N, alpha, static_cast<float*>(C), ldc, shadow, lds));
   LUB_LAUNCH_CHECK();
   return LU_SUCCESS;
 }

@@ -12,7 +12,6 @@ namespace {
 
 __global__ void fill_int_kernel(int* p, int v, int64_t count) {
   dependency_wait();
-  dependents_launch();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < count) p[i] = v;
 }
@@ -82,7 +81,8 @@ cudaError_t set_smem_limit(const void* func, size_t bytes) {
 
 lu_status launch_fill_int(cudaStream_t st, int* p, int v, int64_t count) {
   if (count <= 0) return LU_SUCCESS;
-  LUB_CUDA_TRY(launch_dependent(fill_int_kernel, (unsigned)ceil_div(count, 256), 256, 0, st, p, v, count));
+  LUB_CUDA_TRY(launch_dependent(fill_int_kernel, (unsigned)ceil_div(count, 256), 256, 0, st, p, v,
+                                count));
   LUB_LAUNCH_CHECK();
   return LU_SUCCESS;
 }

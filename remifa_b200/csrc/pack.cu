@@ -162,7 +162,6 @@ pack_a_kernel(int64_t M, int64_t K, const S* __restrict__ src, int64_t lds,
               T* __restrict__ dst, int64_t ldd, int* err) {
   __shared__ float tile[TA * (TA + 1)];  // [k][i]
   dependency_wait();
-  dependents_launch();
   const int64_t i0 = (int64_t)blockIdx.x * TA, k0 = (int64_t)blockIdx.y * TA;
   if (err && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *err = 0;
   float m = 0.0f;
@@ -178,7 +177,6 @@ __global__ void __launch_bounds__(256)
 pack_b_kernel(int64_t K, int64_t N, const S* __restrict__ src, int64_t lds,
               T* __restrict__ dst, int64_t ldd) {
   dependency_wait();
-  dependents_launch();
   const int64_t j = (int64_t)blockIdx.x * kBCols + (threadIdx.x >> 5);
   if (j >= N) return;
   const bool vec = cols_aligned(src, lds);
@@ -228,7 +226,6 @@ pack_scaled_kernel(int nA, int64_t M, int64_t N, int64_t K, int64_t kp,
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   cg::cluster_group cl = cg::this_cluster();
   dependency_wait();
-  dependents_launch();
   cl.barrier_arrive();   // waited for before the first remote store
   const int rank = (int)cl.block_rank();
   const int t = (int)(blockIdx.x / kScaledCtas);
@@ -295,7 +292,8 @@ template <typename T, typename S>
 lu_status pack_a_typed(cudaStream_t st, int64_t M, int64_t K, const S* src,
                        int64_t lds, void* dst, int64_t ldd, int* err = nullptr) {
   dim3 grid((unsigned)ceil_div(M, TA), (unsigned)ceil_div(K, TA));
-  LUB_CUDA_TRY(launch_dependent(pack_a_kernel<T, S>, grid, 256, 0, st, M, K, src, lds, (T*)dst, ldd, err));
+  LUB_CUDA_TRY(launch_dependent(pack_a_kernel<T, S>, grid, 256, 0, st, M, K, src, lds, (T*)dst,
+                                ldd, err));
   LUB_LAUNCH_CHECK();
   return LU_SUCCESS;
 }
@@ -303,7 +301,8 @@ lu_status pack_a_typed(cudaStream_t st, int64_t M, int64_t K, const S* src,
 template <typename T, typename S>
 lu_status pack_b_typed(cudaStream_t st, int64_t K, int64_t N, const S* src,
                        int64_t lds, void* dst, int64_t ldd) {
-  LUB_CUDA_TRY(launch_dependent(pack_b_kernel<T, S>, (unsigned)ceil_div(N, kBCols), 256, 0, st, K, N, src, lds, (T*)dst, ldd));
+  LUB_CUDA_TRY(launch_dependent(pack_b_kernel<T, S>, (unsigned)ceil_div(N, kBCols), 256, 0, st, K,
+                                N, src, lds, (T*)dst, ldd));
   LUB_LAUNCH_CHECK();
   return LU_SUCCESS;
 }
@@ -353,10 +352,14 @@ lu_status launch_pack_scaled(cudaStream_t st, TcOperand kind, int64_t M, int64_t
   const float bound = tc_scale_bound(kind);
   const unsigned grid = (unsigned)(kScaledCtas * (nA + nB));
   if (kind == TcOperand::E4M3) {
-    LUB_CUDA_TRY(launch_dependent(pack_scaled_kernel<uint8_t, false>, grid, 256, 0, st, (int)nA, M, N, K, kp, a, lda, (uint8_t*)da, sa, b, ldb, (uint8_t*)db, sb, ldd, bound));
+    LUB_CUDA_TRY(launch_dependent(pack_scaled_kernel<uint8_t, false>, grid, 256, 0, st, (int)nA,
+                                  M, N, K, kp, a, lda, (uint8_t*)da, sa, b, ldb, (uint8_t*)db, sb,
+                                  ldd, bound));
   } else if (kind == TcOperand::SPLIT16) {
     if (ldd < 3 * kp) return LU_ERR_INVALID_ARG;
-    LUB_CUDA_TRY(launch_dependent(pack_scaled_kernel<__half, true>, grid, 256, 0, st, (int)nA, M, N, K, kp, a, lda, (__half*)da, sa, b, ldb, (__half*)db, sb, ldd, bound));
+    LUB_CUDA_TRY(launch_dependent(pack_scaled_kernel<__half, true>, grid, 256, 0, st, (int)nA, M,
+                                  N, K, kp, a, lda, (__half*)da, sa, b, ldb, (__half*)db, sb, ldd,
+                                  bound));
   } else {
     return LU_ERR_INVALID_ARG;
   }

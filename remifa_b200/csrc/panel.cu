@@ -617,7 +617,6 @@ lupanel_kernel(float* __restrict__ dg, int64_t lda, int w, int64_t M,
                int64_t N, int nL, int64_t offL, int64_t offU, LuPack pk) {
   extern __shared__ __align__(16) float smem[];
   dependency_wait();
-  dependents_launch();
   const int wp = ((w + 7) / 8) * 8;  // padded width (zero filled)
   const int lf = wp + 4;
   // factor block; the update reads 128 columns whatever w is (the positions
@@ -807,7 +806,8 @@ ref_panel_f16_kernel(int64_t m, int n, const __half* __restrict__ d, int64_t ldd
 lu_status launch_diag_factor(cudaStream_t st, float* a, int64_t lda, int w,
                              int64_t col0, int* first_bad) {
   if (w <= 0 || w > 128) return LU_ERR_INVALID_ARG;
-  LUB_CUDA_TRY(launch_dependent(diag_factor_kernel<false>, 1, kDiagThreads, 0, st, a, lda, w, col0, first_bad));
+  LUB_CUDA_TRY(launch_dependent(diag_factor_kernel<false>, 1, kDiagThreads, 0, st, a, lda, w,
+                                col0, first_bad));
   LUB_LAUNCH_CHECK();
   return LU_SUCCESS;
 }
@@ -817,7 +817,8 @@ lu_status launch_diag_crout(cudaStream_t st, float* a, int64_t lda, int w,
   if (w <= 0 || w > 128) return LU_ERR_INVALID_ARG;
   constexpr size_t sm = 128 * kDiagLD * sizeof(float);
   LUB_CUDA_TRY(set_smem_limit((const void*)diag_factor_kernel<true>, sm));
-  LUB_CUDA_TRY(launch_dependent(diag_factor_kernel<true>, 1, kDiagThreads, sm, st, a, lda, w, col0, first_bad));
+  LUB_CUDA_TRY(launch_dependent(diag_factor_kernel<true>, 1, kDiagThreads, sm, st, a, lda, w,
+                                col0, first_bad));
   LUB_LAUNCH_CHECK();
   return LU_SUCCESS;
 }
@@ -829,7 +830,8 @@ static lu_status launch_lupanel_items(cudaStream_t st, float* dg, int64_t lda, i
   const size_t wp = (size_t)((w + 7) / 8) * 8;
   const size_t sm = (128 * (wp + 4) + wp + 2 * 8 * (ITEMS + 4)) * sizeof(float);
   LUB_CUDA_TRY(set_smem_limit((const void*)lupanel_kernel<LEFT, ITEMS>, sm));
-  LUB_CUDA_TRY(launch_dependent(lupanel_kernel<LEFT, ITEMS>, (unsigned)(nL + nU), 8 * ITEMS, sm, st, dg, lda, w, M, N, (int)nL, offL, offU, pk));
+  LUB_CUDA_TRY(launch_dependent(lupanel_kernel<LEFT, ITEMS>, (unsigned)(nL + nU), 8 * ITEMS, sm,
+                                st, dg, lda, w, M, N, (int)nL, offL, offU, pk));
   LUB_LAUNCH_CHECK();
   return LU_SUCCESS;
 }

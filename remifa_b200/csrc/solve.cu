@@ -1105,7 +1105,6 @@ residual_partial_kernel(int64_t n, const float* __restrict__ A, int64_t lda,
                         const double* __restrict__ x, double* __restrict__ P) {
   __shared__ double xs[kRC];
   dependency_wait();
-  dependents_launch();
   const int64_t c0 = (int64_t)blockIdx.y * kRC;
   const int cn = (int)((n - c0) < kRC ? (n - c0) : kRC);
   for (int k = threadIdx.x; k < cn; k += kT) xs[k] = x[c0 + k];
@@ -1178,7 +1177,6 @@ rowsum_final_kernel(int64_t n, int nchunks, const double* __restrict__ P,
 __global__ void axpy_kernel(int64_t n, int64_t nrhs, const double* __restrict__ d,
                             double* __restrict__ x, int64_t ldx) {
   dependency_wait();
-  dependents_launch();
   const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (e < n * nrhs) {
     const int64_t c = e / n;
