@@ -1186,38 +1186,45 @@ __global__ void axpy_kernel(int64_t n, int64_t nrhs, const double* __restrict__ 
 
 
 // ---- residuals of several right-hand sides: R = B - op(A) X on the FP64
-// matrix instruction.  A CTA of eight warps computes RG x 16 rows of R for 8 NF
-// right-hand sides; KS = 8 / RG warps share each 16 rows, each taking its 32 of
-// every 32 KS values of the sum.  A goes straight from global memory to
-// registers (fp32, converted there), one stage of 32 ahead; X is staged in
-// shared memory by cp.async.  The sums' order is fixed, so the result does
-// not depend on scheduling.  maxes[3c .. 3c+2] receive max |r|, |x|, |b| of
-// column c.
+// matrix instruction.  A CTA computes RG x 16 rows of R for 8 NF right-hand
+// sides; KS warps share each 16 rows, each taking its share RK of the KT values
+// of the sum in a stage.  A goes straight from global memory to registers (fp32,
+// converted there), one stage ahead; X is staged in shared memory by cp.async.
+// The next stage's loads are spread over the steps of the current one: issued
+// together after the barrier they held all warps' matrix instructions up.  The
+// sums' order is fixed, so the result does not depend on scheduling.  maxes[3c ..
+// 3c+2] receive max |r|, |x|, |b| of column c.
 //
 // Bound by the FP64 rate from 32 right-hand sides on (n = 8192, 64 columns: 4.3
-// G multiply-adds, 0.24 ms at 64 per cycle and SM), below that by reading A
-// once, for which KS grows as NF shrinks: more, smaller CTAs in flight.  n =
-// 8192, 64 columns on B200: 0.52 ms (transposed 0.47), against 1.20 (1.86)
-// with plain FMAs in groups of 8 columns.
+// G multiply-adds, 0.24 ms at 64 per cycle and SM, 0.28 on the 128 SMs that 64
+// rows per CTA fill), below that by reading A once, for which KS grows as NF
+// shrinks: more, smaller CTAs in flight.  Eight column groups need 16 warps to
+// cover the instruction's latency.  n = 8192, 64 columns on B200: 0.42 ms
+// (transposed 0.37); 0.52 (0.47) with 8 warps and the loads together, 1.20 (1.86)
+// with plain FMAs in groups of 8 columns.  n = 4096 with 32 rows per CTA: 0.139
+// (0.128), against 0.263 (0.237) with 64.
 // Bit pattern of |v|: ordered like the values, NaN above infinity.
 __device__ __forceinline__ unsigned long long abs_bits(double v) {
   return (unsigned long long)__double_as_longlong(fabs(v));
 }
 
-constexpr int kRK = 32;   // values of a sum per warp and stage
+constexpr int residual_kt(int nf) { return nf > 1 ? 512 / nf : 256; }  // values per stage
 
-template <int NF, int KS>
+template <int NF, int KS, int RG>
 constexpr size_t residual_smem() {
-  return (size_t)2 * 8 * NF * (kRK * KS + 4) * sizeof(double);
+  const size_t x = (size_t)2 * 8 * NF * (residual_kt(NF) + 4);   // two stages of X
+  const size_t p = (size_t)(KS - 1) * RG * 32 * 4 * NF;          // partial sums
+  return (x > p ? x : p) * sizeof(double);
 }
 
-template <bool TRANS, int NF, int KS>
-__global__ void __launch_bounds__(kT)
+template <bool TRANS, int NF, int KS, int RG>
+__global__ void __launch_bounds__(32 * KS * RG)
 residual_multi_kernel(int64_t n, int64_t nrhs, const float* __restrict__ A, int64_t lda,
                       const double* __restrict__ B, int64_t ldb,
                       const double* __restrict__ X, int64_t ldx, double* __restrict__ R,
                       int64_t ldr, unsigned long long* __restrict__ maxes) {
-  constexpr int RG = 8 / KS, NC = 8 * NF, KT = kRK * KS;
+  constexpr int NT = 32 * KS * RG, NC = 8 * NF, KT = residual_kt(NF);
+  constexpr int RK = KT / KS, SK = RK / 4;  // values, steps of a warp per stage
   constexpr int S = KT + 4;   // column stride of the X stage: conflict-free fragment reads
   extern __shared__ __align__(16) double xs[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -1238,9 +1245,8 @@ residual_multi_kernel(int64_t n, int64_t nrhs, const float* __restrict__ A, int6
   // entry s of a stage: this lane's k = 4 s + lk, or (transposed) 8 (s / 2) + 2
   // lk + (s & 1), so that a lane reads neighbours; k past n repeats the last
   // one against zeros of X
-  auto load_a = [&](int64_t kb, float (&v)[8][2]) {
-#pragma unroll
-    for (int s = 0; s < 8; s += TRANS ? 2 : 1)
+  auto load_a = [&](int s, int64_t kb, float (&v)[SK][2]) {
+    if (!TRANS || s % 2 == 0)
 #pragma unroll
       for (int m = 0; m < 2; ++m) {
         if (TRANS) {
@@ -1259,16 +1265,23 @@ residual_multi_kernel(int64_t n, int64_t nrhs, const float* __restrict__ A, int6
         }
       }
   };
-  auto load_x = [&](int64_t k0, double* dst) {
-    for (int e = tid; e < NC * KT; e += kT) {
-      const int c = e / KT, k = e % KT;
-      const bool ok = c < nc && k0 + k < n;
-      const double* src = ok ? X + (k0 + k) + (c0 + c) * ldx : X;
-      const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(dst + c * S + k));
-      asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src),
-                   "r"(ok ? 8 : 0) : "memory");
+  // this thread's entries of an X stage: value tid % KT of every (NT / KT)th
+  // column, XE of them, an SKth per step
+  constexpr int XC = NT / KT, XE = NC / XC;
+  static_assert(NT % KT == 0 && XE % SK == 0, "X stage");
+  const int xk = tid % KT, xc = tid / KT;
+  const double* xsrc = X + xk + (c0 + xc) * ldx;
+  const uint32_t xdst = static_cast<uint32_t>(__cvta_generic_to_shared(xs + xc * S + xk));
+  auto load_x = [&](int s, int64_t k0, int buf) {
+    const bool in = k0 + xk < n;
+#pragma unroll
+    for (int e = s * (XE / SK); e < (s + 1) * (XE / SK); ++e) {
+      const bool ok = in && xc + e * XC < nc;
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(
+                       xdst + (uint32_t)((buf * NC + e * XC) * S * 8)),
+                   "l"(ok ? xsrc + k0 + e * XC * ldx : X), "r"(ok ? 8 : 0)
+                   : "memory");
     }
-    trsv::cp_commit();
   };
 
   double acc[2][NF][2];
@@ -1276,22 +1289,22 @@ residual_multi_kernel(int64_t n, int64_t nrhs, const float* __restrict__ A, int6
   for (int m = 0; m < 2; ++m)
 #pragma unroll
     for (int f = 0; f < NF; ++f) acc[m][f][0] = acc[m][f][1] = 0.0;
-  float cur[8][2], nxt[8][2];
-  load_x(0, xs);
-  load_a(kRK * kh, cur);
+  float cur[SK][2], nxt[SK][2];
+#pragma unroll
+  for (int s = 0; s < SK; ++s) {
+    load_x(s, 0, 0);
+    load_a(s, RK * kh, cur);
+  }
+  trsv::cp_commit();
   const int nst = (int)((n + KT - 1) / KT);
 #pragma unroll 1
   for (int t = 0; t < nst; ++t) {
     const int64_t k1 = (int64_t)(t + 1) * KT;
     trsv::cp_wait<0>();
     __syncthreads();  // stage t is in, stage t - 1 read
-    if (t + 1 < nst) {
-      load_x(k1, xs + ((t + 1) & 1) * NC * S);
-      load_a(k1 + kRK * kh, nxt);
-    }
-    const double* x = xs + (t & 1) * NC * S + lr * S + kRK * kh;
+    const double* x = xs + (t & 1) * NC * S + lr * S + RK * kh;
 #pragma unroll
-    for (int s = 0; s < 8; ++s) {
+    for (int s = 0; s < SK; ++s) {
       const int k = TRANS ? 8 * (s >> 1) + 2 * lk + (s & 1) : 4 * s + lk;
       const double a0 = (double)cur[s][0], a1 = (double)cur[s][1];
 #pragma unroll
@@ -1300,9 +1313,14 @@ residual_multi_kernel(int64_t n, int64_t nrhs, const float* __restrict__ A, int6
         mma64(acc[0][f], a0, b);
         mma64(acc[1][f], a1, b);
       }
+      if (t + 1 < nst) {  // the next stage, spread over the steps
+        load_x(s, k1, (t + 1) & 1);
+        load_a(s, k1 + RK * kh, nxt);
+      }
     }
+    trsv::cp_commit();
 #pragma unroll
-    for (int s = 0; s < 8; ++s) {
+    for (int s = 0; s < SK; ++s) {
       cur[s][0] = nxt[s][0];
       cur[s][1] = nxt[s][1];
     }
@@ -1359,16 +1377,16 @@ residual_multi_kernel(int64_t n, int64_t nrhs, const float* __restrict__ A, int6
     }
 }
 
-template <bool TRANS, int NF, int KS>
+template <bool TRANS, int NF, int KS, int RG>
 lu_status launch_residual_as(cudaStream_t st, int64_t n, int64_t nrhs, const float* A,
                              int64_t lda, const double* B, int64_t ldb, const double* X,
                              int64_t ldx, double* R, int64_t ldr, unsigned long long* maxes) {
   const int64_t groups = ceil_div(nrhs, 8 * NF);
   if (groups > 65535) return LU_ERR_INVALID_ARG;
-  dim3 g((unsigned)ceil_div(n, 16 * (8 / KS)), (unsigned)groups);
-  LUB_CUDA_TRY(set_smem_limit((const void*)residual_multi_kernel<TRANS, NF, KS>,
-                              residual_smem<NF, KS>()));
-  residual_multi_kernel<TRANS, NF, KS><<<g, kT, residual_smem<NF, KS>(), st>>>(
+  dim3 g((unsigned)ceil_div(n, 16 * RG), (unsigned)groups);
+  constexpr size_t sm = residual_smem<NF, KS, RG>();
+  LUB_CUDA_TRY(set_smem_limit((const void*)residual_multi_kernel<TRANS, NF, KS, RG>, sm));
+  residual_multi_kernel<TRANS, NF, KS, RG><<<g, 32 * KS * RG, sm, st>>>(
       n, nrhs, A, lda, B, ldb, X, ldx, R, ldr, maxes);
   LUB_LAUNCH_CHECK();
   return LU_SUCCESS;
@@ -1379,10 +1397,13 @@ template <bool TRANS>
 lu_status launch_residual_nf(cudaStream_t st, int64_t n, int64_t nrhs, const float* A,
                              int64_t lda, const double* B, int64_t ldb, const double* X,
                              int64_t ldx, double* R, int64_t ldr, unsigned long long* maxes) {
-  const auto fn = nrhs <= 8    ? launch_residual_as<TRANS, 1, 8>
-                  : nrhs <= 16 ? launch_residual_as<TRANS, 2, 8>
-                  : nrhs <= 32 ? launch_residual_as<TRANS, 4, 4>
-                               : launch_residual_as<TRANS, 8, 2>;
+  // 32 rows per CTA while that is one wave
+  const bool few = n <= 32 * (int64_t)sm_count();
+  const auto fn = nrhs <= 8    ? launch_residual_as<TRANS, 1, 8, 1>
+                  : nrhs <= 16 ? launch_residual_as<TRANS, 2, 8, 1>
+                  : nrhs <= 32 ? launch_residual_as<TRANS, 4, 4, 2>
+                  : few        ? launch_residual_as<TRANS, 8, 8, 2>
+                               : launch_residual_as<TRANS, 8, 4, 4>;
   return fn(st, n, nrhs, A, lda, B, ldb, X, ldx, R, ldr, maxes);
 }
 }  // namespace
