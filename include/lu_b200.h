@@ -393,8 +393,8 @@ LU_API void lu_batch_graph_destroy(lu_batch_graph graph);
  * n_i x nrhs, ld n_i) holds B_i on entry and X_i = op(A_i)^-1 B_i on exit
  * (trans = 1: A_i^T).  fp32 factors d_lu[i] (ld d_ldlu[i], NULL: n_i), fp64
  * arithmetic; with the original matrices d_a (ld d_lda, NULL: n_i) each
- * column then gets refine_iters rounds of FP64 refinement.  One warp per
- * (matrix, column), no allocation, asynchronous. */
+ * column then gets refine_iters rounds of FP64 refinement.  One CTA per
+ * matrix, no allocation, asynchronous. */
 LU_API lu_status lu_batch_solve_c(lu_batch_plan plan, lu_stream_t stream,
                                   const float* const* d_lu, const int32_t* d_ldlu,
                                   const float* const* d_a, const int32_t* d_lda,
