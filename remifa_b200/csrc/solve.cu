@@ -10,8 +10,8 @@
 // factorization error -- what iterative refinement in fp64 needs.
 //
 // op(T) X = B, T = L (unit lower) or U (upper), op = identity or transpose,
-// runs as one launch per triangle after a copy kernel that moves B aside and
-// marks every entry of X pending (a signalling-NaN pattern no arithmetic
+// runs as one launch per triangle after a kernel that marks every entry of the
+// solution pending, one for both triangles (a signalling-NaN pattern no arithmetic
 // produces).  A CTA per (row block of 64 rows, group of 1, 2 or 8 right-hand
 // sides); CTAs draw tickets in solve order (an atomic counter), so a CTA only
 // ever waits for CTAs already running: no deadlock whatever the residency.
@@ -23,9 +23,9 @@
 // Dinv op(T)[t, t-1] while the CTA waits, so the hand-over from block t-1 to
 // block t is, per warp and without a CTA barrier: x_t = Dinv (b -
 // sum_{q<t-1} op(T)[t,q] x_q) - W x_{t-1}.  trsv_kernel does this with FMAs
-// and shuffles for 1 or 2 right-hand sides, trsv_mma_kernel on the FP64 matrix
+// and shuffles for 1 to 4 right-hand sides (groups of 1 or 2), trsv_mma_kernel on the FP64 matrix
 // instruction for groups of 8.  On B200: one right-hand side, n = 10007, L and U
-// 0.293 ms (0.344 without clusters), n = 16384 0.475 (0.573); 64 right-hand
+// 0.278 ms (0.344 without clusters), n = 16384 0.46 (0.58); 64 right-hand
 // sides, n = 8192 0.82 (1.36 with a counter per group and shared-memory
 // tiles).  Bound by the chain of n / 64 hand-overs.
 #include "common.cuh"
@@ -290,7 +290,6 @@ __host__ __device__ constexpr size_t warp_smem_bytes(int nr) {
   return (size_t)S * 8 * kWarpTile * 4    // per-warp tile rings (fp32)
          + (size_t)BS * BS * 8            // inverse of the diagonal block (fp64)
          + (size_t)BS * BS * 4            // tile of the previous block (fp32)
-         + (size_t)8 * nr * BS * 8        // per-warp partial sums
          + (size_t)BS * 8                 // reciprocals of the diagonal
          + (size_t)kCluster * nr * BS * 8 // solutions of the cluster's blocks
          + 64;                            // control words
@@ -531,8 +530,7 @@ trsv_kernel(Args a) {
   float* ring = reinterpret_cast<float*>(smem);
   double* Dinv = reinterpret_cast<double*>(smem + (size_t)S * 8 * kWarpTile * 4);
   float* Tw = reinterpret_cast<float*>(Dinv + BS * BS);
-  double* part = reinterpret_cast<double*>(Tw + BS * BS);
-  double* rdiag = part + 8 * NR * BS;
+  double* rdiag = reinterpret_cast<double*>(Tw + BS * BS);
   double* xin = rdiag + BS;              // [block of the cluster][column][row]
   int* ctrl = reinterpret_cast<int*>(xin + kCluster * NR * BS);
 
@@ -721,6 +719,9 @@ trsv_kernel(Args a) {
     fetch_x<2, NR>(xf, a, tile_k0(t - 1), tile_kw(t - 1), c0, nc, lane, 32);
 
   // ---- partial sums of the warps -> y = b - sum -> c = Dinv y ----
+  // (each in its warp's ring, which is done with: two CTAs fit on an SM)
+  auto part = [&](int w) { return reinterpret_cast<double*>(ring + w * S * kWarpTile); };
+  __syncwarp();
   if (TRANS) {
 #pragma unroll
     for (int c = 0; c < NR; ++c) {
@@ -728,13 +729,13 @@ trsv_kernel(Args a) {
 #pragma unroll
       for (int i = 0; i < 8; ++i) v[i] = acc[i][c];
       const double s = row_reduce(v, lane);
-      if ((lane & 3) == 0) part[c * BS + 8 * warp + (lane >> 2)] = s;
+      if ((lane & 3) == 0) part(warp)[c * 8 + (lane >> 2)] = s;
     }
   } else {
 #pragma unroll
     for (int c = 0; c < NR; ++c)
 #pragma unroll
-      for (int h = 0; h < 2; ++h) part[(warp * NR + c) * BS + lane + 32 * h] = acc[h][c];
+      for (int h = 0; h < 2; ++h) part(warp)[c * BS + lane + 32 * h] = acc[h][c];
   }
   __syncthreads();
   double cv[NR];
@@ -746,11 +747,11 @@ trsv_kernel(Args a) {
       const int m = lane + 32 * h;
       double s;
       if (TRANS) {
-        s = part[c * BS + m];
+        s = part(m >> 3)[c * 8 + (m & 7)];
       } else {
-        s = part[c * BS + m];
+        s = part(0)[c * BS + m];
 #pragma unroll
-        for (int w = 1; w < 8; ++w) s += part[(w * NR + c) * BS + m];
+        for (int w = 1; w < 8; ++w) s += part(w)[c * BS + m];
       }
       y[h] = bm[h][c] - s;
     }
@@ -1033,15 +1034,20 @@ trsv_mma_kernel(Args a) {
       st_publish(a.X + (r0 + row) + (c0 + 2 * lk + h) * a.ldx, cv[0][h]);
 }
 
-// Right-hand sides per CTA: from three on, the matrix kernel's 8.
-int group_width(int64_t nrhs) { return nrhs >= 3 ? 8 : nrhs == 2 ? 2 : 1; }
+// Right-hand sides per CTA: from five on, the matrix kernel's 8; three or four as
+// two groups of two (three, on B200: n = 2000 100 us, 8192 329, 10007 569, against
+// 126, 464 and 636 with the matrix kernel; five would take 100, 482 and 862 in
+// pairs, 132, 498 and 703 with the matrix kernel).
+int group_width(int64_t nrhs) { return nrhs >= 5 ? 8 : nrhs >= 2 ? 2 : 1; }
 
 template <bool TRANS, int NR, bool V16>
 lu_status launch_one(cudaStream_t st, const Args& a) {
   size_t smem;
   void (*fn)(Args);
   if constexpr (NR <= 2) {
-    smem = warp_smem_bytes(NR);
+    // one group of two has the SMs for itself: a CTA each (n = 10007 409 us; 469
+    // with two to an SM).  Two groups share them.
+    smem = warp_smem_bytes(NR) + (NR == 2 && a.ngroups == 1 ? (size_t)8 * NR * BS * 8 : 0);
     fn = trsv_kernel<TRANS, NR, V16>;
     LUB_CUDA_TRY(set_smem_limit((const void*)fn, smem));
     // clusters of more than 8 CTAs are allowed per kernel, once per device
