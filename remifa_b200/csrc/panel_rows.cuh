@@ -148,7 +148,8 @@ __device__ __forceinline__ void update_block(float* X, const float* Lp, const fl
 // 4 with at least three rows of padding, 64 columns allocated: the update's
 // blocks reach past row n and column wj).  inv: 8 floats (16-byte aligned) in
 // shared memory; zero / non-finite pivots are reported to *bad as 1-based
-// column pbase + k.
+// column pbase + k.  Ends with a CTA barrier on every path: the caller reads the
+// block with another thread-to-row mapping.
 template <int NT>
 __device__ __forceinline__ void panel_block(float* C, int ldc, int n, int c0, int wj,
                                             float* inv, int* bad, int pbase) {
@@ -171,8 +172,8 @@ __device__ __forceinline__ void panel_block(float* C, int ldc, int n, int c0, in
       const int c = t1 + (NT - 1 - tid);     // the last warps: free of rows in small blocks
       if (c < wj) eliminate_column(P + t0 + c * ldc, T, ldc);
     }
-    if (t + 1 == nt) break;
     __syncthreads();
+    if (t + 1 == nt) break;
     if (warp == 0) {
       const int tw = min(8, wj - t1);
       float* N = P + t1 + t1 * ldc;
