@@ -11,9 +11,10 @@
 //   diag_factor_kernel : the w x w diagonal block, one CTA, in registers (with
 //                        the left-looking variant's Crout order as an option);
 //   lupanel_kernel     : the L21 rows below the block and the U12 columns
-//                        right of it, 64 rows or 64 columns per CTA (one grid
-//                        for both strips), optionally writing the K-major
+//                        right of it, 32 or 64 rows or columns per CTA (one
+//                        grid for both strips), optionally writing the K-major
 //                        tensor-core operand copies of what it finishes;
+//   lupanel_wide_kernel: the same for large right-looking launches;
 //   ref_panel_kernel   : remifa::lu_nopiv_panel<float,8> as a standalone
 //                        entry point (lu_panel_c);
 // each replaying, per element, the reference's exact operation sequence
@@ -391,7 +392,7 @@ diag_factor_kernel(float* __restrict__ a, int64_t lda, int w, int64_t col0,
 // ---------------------------------------------------------------------------
 // L and U panels of one sub-panel, one launch.  `dg` is the factored w x w
 // diagonal block (lda); M rows lie below it (L21), N columns right of it
-// (U12).  A CTA owns kItems rows of L21 or columns of U12 ("items") of w
+// (U12).  A CTA owns ITEMS rows of L21 or columns of U12 ("items") of w
 // positions each, and walks the 8-wide tiles t left to right:
 //   (a) one thread per item eliminates tile t of its item: L rows
 //       x_k *= 1/d_k, x_j -= x_k U[k][j] (src/lu_nopiv.cu:141-168); U
@@ -409,14 +410,13 @@ diag_factor_kernel(float* __restrict__ a, int64_t lda, int w, int64_t col0,
 // The items live in registers: thread (tx, ty) holds items 4 tx .. 4 tx + 3 at
 // positions 4 ty .. 4 ty + 3, so the update reads only the tile's item strip
 // and the factor values from shared memory and writes nothing back, and the
-// warps left of the current tile drop out.  Large launches (64 items per CTA)
-// are bounded by the FMA and shared-memory read rates, small ones (32) by the
-// chain of w / 8 tiles.  w = 128 on B200, launches back to back, items of
-// both strips: 256: 12.5 us (16.6 with the items in shared memory), 8192:
-// 18.7 (18.7), 27648: 39 (40).
-
-// rows / columns per CTA: 64, or 32 where that still fills less than a wave
-// (a shorter chain); 8 threads per item
+// warps left of the current tile drop out.  8 threads per item, 32 items per CTA
+// where that is at most one CTA per SM -- bound by the chain of w / 8 tiles; w =
+// 128 on B200, launches back to back, 256 items of both strips 12.5 us, 16.6 with
+// the items in shared memory -- and 64 in larger left-looking launches, bound by
+// the FMA and shared-memory read rates (fp16 storage, n = 8192: 4.33 ms, 4.48 with
+// lupanel_wide_kernel and the running sums in shared memory).  Larger
+// right-looking launches are lupanel_wide_kernel's.
 
 // What one CTA works on: its items (row i: a + i, column i: a + i * lda) and
 // the factor values that multiply item value k for position p, both as they
@@ -657,6 +657,347 @@ lupanel_kernel(float* __restrict__ dg, int64_t lda, int w, int64_t M,
 }
 
 // ---------------------------------------------------------------------------
+// The right-looking panels of large launches: 64 items per CTA of 256 threads, in
+// shared memory (S[item][pos]).  The item threads eliminate tile T+1 while the
+// other warps still apply tile T's update (one barrier per tile), and the results
+// leave at the end, whole rows of the operand copies at a time.  Alone it takes as
+// long as the register variant with 64 items (27648 items 39 us); beside the bulk
+// update it is the faster one: whole factorizations on B200 with the register
+// variant / this, n = 8192 e4m3 4.11 / 3.83 ms, n = 16384 9.88 / 9.17, n = 24576
+// 23.0 / 21.7, n = 32768 46.8 / 44.2.
+constexpr int kWideThreads = 256;
+constexpr int kWideItems = 64;             // rows / columns per CTA
+constexpr int kMicroI = 4, kMicroP = 8;    // register micro-tile
+
+// Block copies between global memory and shared memory, by all threads
+// of the CTA: warps take columns, lanes consecutive rows, so no index is
+// divided by a runtime extent.  Both sides column-major unless noted.
+
+// dst[r + c*ldd] = src[r + c*lds] asynchronously (complete with
+// cp_async_wait_all); 16-byte copies when every column start is 16-byte
+// aligned on both sides.
+__device__ __forceinline__ void stage_cols_async(float* dst, int ldd, const float* src,
+                                                 int64_t lds, int rows, int cols) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  constexpr int kNW = kWideThreads / 32;
+  const bool vec = ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15) == 0 &&
+                   (lds & 3) == 0 && (ldd & 3) == 0 && (rows & 3) == 0;
+  if (vec) {
+    for (int c = warp; c < cols; c += kNW) {
+      const float* s = src + (int64_t)c * lds;
+      float* d = dst + c * ldd;
+      for (int r = 4 * lane; r < rows; r += 128) cp_async16(d + r, s + r);
+    }
+  } else {
+    for (int c = warp; c < cols; c += kNW) {
+      const float* s = src + (int64_t)c * lds;
+      float* d = dst + c * ldd;
+      for (int r = lane; r < rows; r += 32) cp_async4(d + r, s + r);
+    }
+  }
+}
+
+// dst[r + c*ldd] = src[r + c*lds] (shared -> global), 16-byte stores when
+// every column start is 16-byte aligned on both sides.
+__device__ __forceinline__ void store_cols(float* dst, int64_t ldd, const float* src,
+                                           int lds, int rows, int cols) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  constexpr int kNW = kWideThreads / 32;
+  const bool vec = ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15) == 0 &&
+                   (ldd & 3) == 0 && (lds & 3) == 0 && (rows & 3) == 0;
+  if (vec) {
+    for (int c = warp; c < cols; c += kNW) {
+      const float* s = src + c * lds;
+      float* d = dst + (int64_t)c * ldd;
+      for (int r = 4 * lane; r < rows; r += 128)
+        *reinterpret_cast<float4*>(d + r) = *reinterpret_cast<const float4*>(s + r);
+    }
+  } else {
+    for (int c = warp; c < cols; c += kNW) {
+      const float* s = src + c * lds;
+      float* d = dst + (int64_t)c * ldd;
+      for (int r = lane; r < rows; r += 32) d[r] = s[r];
+    }
+  }
+}
+
+// Transposing load: dst[r*ldd + c] = src[r + c*lds] for r < rows, c < cols,
+// and 0 for cols <= c < round4(cols).  Each thread reads four columns of
+// one row (coalesced across the lanes) and writes them as one 16-byte
+// shared store; dst 16-byte aligned, ldd % 4 == 0.
+__device__ __forceinline__ void stage_rows_t(float* dst, int ldd, const float* src,
+                                             int64_t lds, int rows, int cols) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  constexpr int kNW = kWideThreads / 32;
+  const int nq = (cols + 3) >> 2;
+  for (int q = warp; q < nq; q += kNW) {
+    const int c0 = 4 * q;
+    const float* s = src + (int64_t)c0 * lds;
+#pragma unroll 2
+    for (int r = lane; r < rows; r += 32) {
+      float v[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) v[e] = (c0 + e < cols) ? s[r + e * lds] : 0.0f;
+      *reinterpret_cast<float4*>(dst + r * ldd + c0) = make_float4(v[0], v[1], v[2], v[3]);
+    }
+  }
+}
+
+// Transposing store: dst[r + c*ldd] = src[r*lds + c] for r < rows,
+// c < cols (16-byte shared reads; src 16-byte aligned, lds % 4 == 0).
+__device__ __forceinline__ void store_rows_t(float* dst, int64_t ldd, const float* src,
+                                             int lds, int rows, int cols) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  constexpr int kNW = kWideThreads / 32;
+  const int nq = (cols + 3) >> 2;
+  for (int q = warp; q < nq; q += kNW) {
+    const int c0 = 4 * q;
+    float* d = dst + (int64_t)c0 * ldd;
+#pragma unroll 2
+    for (int r = lane; r < rows; r += 32) {
+      const float4 v4 = *reinterpret_cast<const float4*>(src + r * lds + c0);
+      const float v[4] = {v4.x, v4.y, v4.z, v4.w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (c0 + e < cols) d[r + e * ldd] = v[e];
+    }
+  }
+}
+
+// Eliminate tile columns [t0, t0 + tw) of one item held in x[0..8):
+// L rows x_c -= x_k U[k][c] (k < c), then x_c *= 1/d_c
+// (src/lu_nopiv.cu:141-168); U columns x_c -= L[c][k] x_k
+// (src/lu_nopiv.cu:304-316).
+template <bool IS_L>
+__device__ __forceinline__ void wide_elim(const float* F, int lf, const float* inv,
+                                          int t0, int tw, float (&x)[8]) {
+  if (tw == 8) {
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      float f[8];
+      ld8(F + (t0 + c) * lf + t0, f);  // f[k] = U[k][c] (L) / L[c][k] (U)
+      if (IS_L) {
+#pragma unroll
+        for (int k = 0; k < c; ++k) x[c] = __fmaf_rn(-x[k], f[k], x[c]);
+        x[c] = __fmul_rn(x[c], inv[t0 + c]);
+      } else {
+#pragma unroll
+        for (int k = 0; k < c; ++k) x[c] = __fmaf_rn(-f[k], x[k], x[c]);
+      }
+    }
+  } else {
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      if (c < tw) {
+        const float* f = F + (t0 + c) * lf + t0;
+        if (IS_L) {
+#pragma unroll
+          for (int k = 0; k < c; ++k) x[c] = __fmaf_rn(-x[k], f[k], x[c]);
+          x[c] = __fmul_rn(x[c], inv[t0 + c]);
+        } else {
+#pragma unroll
+          for (int k = 0; k < c; ++k) x[c] = __fmaf_rn(-f[k], x[k], x[c]);
+        }
+      }
+    }
+  }
+}
+
+// F[pos * lf + k]: the factor values that multiply item value k for
+// position pos -- U[k][pos] (L blocks, F column-major) or L[pos][k] (U
+// blocks, F row-major) -- so the 8 values of one tile are two float4.
+// Per tile T, after one barrier:
+//   warps 0-1 (one thread per item) apply tile T's rank-8 update to the
+//     8 positions of tile T+1 and eliminate tile T+1 at once (look-ahead);
+//   warps 2-7 apply tile T's rank-8 update to the positions right of tile
+//     T+1 in register micro-tiles of 4 items x 8 positions (256 FMAs per 24
+//     vector loads).
+// Every element still receives acc = sum_k fma(x_k, F_k) over the tile's 8
+// columns in k order, then one subtraction.
+template <bool IS_L>
+__device__ __forceinline__ void wide_strip(const float* F, int lf, const float* inv,
+                                           float* S, int ls, int w) {
+  constexpr int kIG = kWideItems / kMicroI;  // 16 item groups
+  const int tid = threadIdx.x;
+  const int nt = (w + 7) / 8;
+  if (tid < kWideItems) {  // tile 0
+    float* xr = S + tid * ls;
+    float x[8];
+    ld8(xr, x);
+    wide_elim<IS_L>(F, lf, inv, 0, min(8, w), x);
+    st8(xr, x);
+  }
+  __syncthreads();
+  for (int T = 0; T + 1 < nt; ++T) {
+    const int t0 = 8 * T, p0 = t0 + 8;
+    if (tid < kWideItems) {
+      float* xr = S + tid * ls;
+      float xv[8], x[8], acc[8];
+      ld8(xr + t0, xv);
+      ld8(xr + p0, x);
+#pragma unroll
+      for (int b = 0; b < 8; ++b) acc[b] = 0.0f;
+#pragma unroll
+      for (int b = 0; b < 8; ++b) {
+        float f[8];
+        ld8(F + (p0 + b) * lf + t0, f);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) acc[b] = __fmaf_rn(xv[k], f[k], acc[b]);
+      }
+#pragma unroll
+      for (int b = 0; b < 8; ++b) x[b] = __fsub_rn(x[b], acc[b]);
+      wide_elim<IS_L>(F, lf, inv, p0, min(8, w - p0), x);
+      st8(xr + p0, x);
+    } else {
+      const int q0 = p0 + 8;
+      const int npos = (w - q0 + kMicroP - 1) / kMicroP;
+      for (int m = tid - kWideItems; m < npos * kIG; m += kWideThreads - kWideItems) {
+        const int ig = m % kIG, pp = q0 + (m / kIG) * kMicroP;
+        float xv[kMicroI][8];
+#pragma unroll
+        for (int a = 0; a < kMicroI; ++a) ld8(S + (ig + a * kIG) * ls + t0, xv[a]);
+        float acc[kMicroI][kMicroP];
+#pragma unroll
+        for (int a = 0; a < kMicroI; ++a)
+#pragma unroll
+          for (int b = 0; b < kMicroP; ++b) acc[a][b] = 0.0f;
+#pragma unroll
+        for (int b = 0; b < kMicroP; ++b) {
+          float f[8];
+          ld8(F + (pp + b) * lf + t0, f);
+#pragma unroll
+          for (int k = 0; k < 8; ++k)
+#pragma unroll
+            for (int a = 0; a < kMicroI; ++a) acc[a][b] = __fmaf_rn(xv[a][k], f[k], acc[a][b]);
+        }
+#pragma unroll
+        for (int a = 0; a < kMicroI; ++a) {
+          float* row = S + (ig + a * kIG) * ls + pp;
+          float c[8];
+          ld8(row, c);
+#pragma unroll
+          for (int b = 0; b < kMicroP; ++b) c[b] = __fsub_rn(c[b], acc[a][b]);
+          st8(row, c);
+        }
+      }
+    }
+    __syncthreads();
+  }
+}
+
+__global__ void __launch_bounds__(kWideThreads)
+lupanel_wide_kernel(float* __restrict__ dg, int64_t lda, int w, int64_t M,
+               int64_t N, int nL, int64_t offL, int64_t offU, LuPack pk) {
+  extern __shared__ __align__(16) float smem[];
+  const int tid = threadIdx.x;
+  dependency_wait();
+  const int wp = ((w + 7) / 8) * 8;  // padded width (zero filled)
+  const int ls = wp + 4;             // item stride (breaks bank aliasing)
+  const int lf = wp + 4;             // leading dimension of F, same reason
+  float* F = smem;                   // diagonal block, wp x wp
+  float* inv = F + (size_t)wp * lf;  // wp
+  float* S = inv + wp;               // kWideItems x ls
+  const bool is_l = (int)blockIdx.x < nL;
+
+  // Stage the factored diagonal block: column-major (F[c*lf + r]) for L
+  // blocks, row-major (F[r*lf + c]) for U blocks; the padding rows and
+  // columns [w, wp) are zero.
+  if (is_l) stage_cols_async(F, lf, dg, lda, w, w);
+  else stage_rows_t(F, lf, dg, lda, w, w);
+  if (wp != w) {
+    for (int idx = tid; idx < wp * wp; idx += kWideThreads) {
+      const int r = idx % wp, c = idx / wp;
+      if (r >= w || c >= (is_l ? w : ((w + 3) & ~3))) F[is_l ? c * lf + r : r * lf + c] = 0.0f;
+    }
+  }
+  int64_t item0;
+  float* A;
+  int nitems;
+  if (is_l) {
+    item0 = (int64_t)blockIdx.x * kWideItems;
+    A = dg + w + offL;               // first row of this launch's L rows
+    nitems = (int)std::min<int64_t>(kWideItems, M - item0);
+    // S[q*ls + c] = A[row item0 + q, column c]
+    stage_rows_t(S, ls, A + item0, lda, nitems, w);
+  } else {
+    item0 = (int64_t)(blockIdx.x - nL) * kWideItems;
+    A = dg + (w + offU) * lda;       // first column of this launch's U columns
+    nitems = (int)std::min<int64_t>(kWideItems, N - item0);
+    // S[q*ls + i] = A[row i, column item0 + q]
+    stage_cols_async(S, ls, A + item0 * lda, lda, w, nitems);
+  }
+  // zero the positions [w, wp) of every item and the items past the end
+  {
+    const int wq = is_l ? ((w + 3) & ~3) : w;  // the L staging zeroed up to round4(w)
+    const int padc = wp - wq;
+    if (padc > 0)
+      for (int idx = tid; idx < kWideItems * padc; idx += kWideThreads)
+        S[(idx / padc) * ls + wq + idx % padc] = 0.0f;
+    for (int idx = nitems * ls + tid; idx < kWideItems * ls; idx += kWideThreads) S[idx] = 0.0f;
+  }
+  cp_async_wait_all();
+  __syncthreads();
+  if (is_l) {
+    for (int k = tid; k < wp; k += kWideThreads)
+      inv[k] = (k < w) ? rcp_rn(F[k * lf + k]) : 0.0f;
+    __syncthreads();
+    wide_strip<true>(F, lf, inv, S, ls, w);
+  } else {
+    wide_strip<false>(F, lf, inv, S, ls, w);
+  }
+  if (is_l) store_rows_t(A + item0, lda, S, ls, nitems, w);
+  else store_cols(A + item0 * lda, lda, S, ls, w, nitems);
+  // the finished items as tensor-core operands: item qq's w values are
+  // contiguous along K in both copies (consecutive threads, consecutive k)
+  // destination 0: the tensor-core operand copy; 1: the second L copy
+  for (int dsel = 0; dsel < 2; ++dsel) {
+    void* dst = dsel == 0 ? (is_l ? pk.pa : pk.pb) : (is_l ? pk.pa2 : nullptr);
+    if (!dst) continue;
+    const int64_t lim = is_l ? M : N;
+    const int64_t base = (dsel == 1 ? pk.row02 : is_l ? pk.row0 : pk.col0) + item0;
+    const int64_t ldk = dsel == 1 ? pk.ldk2 : pk.ldk;
+    const int k0 = dsel == 1 ? pk.k02 : pk.k0;
+    if (w % 8 == 0 && ldk % 8 == 0 && k0 % 8 == 0) {
+      // 8 values -> one 16-byte store
+      const int w8 = w / 8;  // <= 16
+      for (int idx = tid; idx < kWideItems * 16; idx += kWideThreads) {
+        const int c8 = idx & 15, qq = idx >> 4;
+        const int64_t pr = base + qq;
+        if (c8 < w8 && item0 + qq < lim && pr >= 0) {
+          float v[8];
+          ld8(&S[qq * ls + 8 * c8], v);
+          uint4 out;
+          uint32_t* o32 = reinterpret_cast<uint32_t*>(&out);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            if (pk.bf16) {
+              const __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * e], v[2 * e + 1]);
+              o32[e] = *reinterpret_cast<const uint32_t*>(&h);
+            } else {
+              const __half2 h = __floats2half2_rn(v[2 * e], v[2 * e + 1]);
+              o32[e] = *reinterpret_cast<const uint32_t*>(&h);
+            }
+          }
+          *reinterpret_cast<uint4*>(static_cast<uint16_t*>(dst) + pr * ldk + k0 + 8 * c8) = out;
+        }
+      }
+    } else {
+      for (int idx = tid; idx < kWideItems * w; idx += kWideThreads) {
+        const int c = idx % w, qq = idx / w;
+        const int64_t pr = base + qq;
+        if (item0 + qq < lim && pr >= 0) {
+          const float v = S[qq * ls + c];
+          const int64_t o = pr * ldk + k0 + c;
+          if (pk.bf16) static_cast<__nv_bfloat16*>(dst)[o] = __float2bfloat16_rn(v);
+          else static_cast<__half*>(dst)[o] = __float2half_rn(v);
+        }
+      }
+    }
+  }
+  (void)nitems;
+}
+
+// ---------------------------------------------------------------------------
 // Reference-compatible panel (remifa::lu_nopiv_panel<float,8>): n <= 8
 // columns, the diagonal tile factored from the copy d by every CTA.
 // blockIdx.y == 0: L rows [n, m); blockIdx.y == 1: U columns [n, m).
@@ -836,6 +1177,18 @@ static lu_status launch_lupanel_items(cudaStream_t st, float* dg, int64_t lda, i
   return LU_SUCCESS;
 }
 
+static lu_status launch_lupanel_wide(cudaStream_t st, float* dg, int64_t lda, int w, int64_t M,
+                                     int64_t N, int64_t offL, int64_t offU, const LuPack& pk) {
+  const int64_t nL = ceil_div(M, kWideItems), nU = ceil_div(N, kWideItems);
+  const size_t wp = (size_t)((w + 7) / 8) * 8;
+  const size_t sm = (wp * (wp + 4) + wp + (size_t)kWideItems * (wp + 4)) * sizeof(float);
+  LUB_CUDA_TRY(set_smem_limit((const void*)lupanel_wide_kernel, sm));
+  LUB_CUDA_TRY(launch_dependent(lupanel_wide_kernel, (unsigned)(nL + nU), kWideThreads, sm, st, dg,
+                                lda, w, M, N, (int)nL, offL, offU, pk));
+  LUB_LAUNCH_CHECK();
+  return LU_SUCCESS;
+}
+
 lu_status launch_lupanel(cudaStream_t st, float* dg, int64_t lda, int w,
                          int64_t M, int64_t N, bool left, int64_t offL, int64_t offU,
                          const LuPack* pack) {
@@ -847,8 +1200,9 @@ lu_status launch_lupanel(cudaStream_t st, float* dg, int64_t lda, int w,
   // 32 items per CTA (a shorter chain per tile) while that is at most one CTA
   // per SM, else 64 (half the reads of the block)
   const bool small = ceil_div(M, 32) + ceil_div(N, 32) <= sm_count();
-  const auto fn = left ? (small ? launch_lupanel_items<true, 32> : launch_lupanel_items<true, 64>)
-                       : (small ? launch_lupanel_items<false, 32> : launch_lupanel_items<false, 64>);
+  const auto fn = left    ? (small ? launch_lupanel_items<true, 32> : launch_lupanel_items<true, 64>)
+                  : small ? launch_lupanel_items<false, 32>
+                          : launch_lupanel_wide;
   return fn(st, dg, lda, w, M, N, offL, offU, pk);
 }
 
