@@ -394,7 +394,7 @@ LU_API void lu_batch_graph_destroy(lu_batch_graph graph);
  * (trans = 1: A_i^T).  fp32 factors d_lu[i] (ld d_ldlu[i], NULL: n_i), fp64
  * arithmetic; with the original matrices d_a (ld d_lda, NULL: n_i) each
  * column then gets refine_iters rounds of FP64 refinement.  One CTA per
- * matrix, no allocation, asynchronous. */
+ * matrix, or one warp per column of a small one; no allocation, asynchronous. */
 LU_API lu_status lu_batch_solve_c(lu_batch_plan plan, lu_stream_t stream,
                                   const float* const* d_lu, const int32_t* d_ldlu,
                                   const float* const* d_a, const int32_t* d_lda,

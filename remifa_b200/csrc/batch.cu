@@ -590,6 +590,7 @@ struct lu_batch_plan_t {
   int nmax = 0;
   std::vector<int32_t> h_n;
   std::vector<int32_t> h_order;
+  std::vector<int32_t> h_upto;  // [n]: matrices of size <= n
   lu_batch_tuning tuning{};
   int32_t* d_n = nullptr;
   int32_t* d_order = nullptr;
@@ -608,6 +609,7 @@ namespace lub {
 int64_t batch_plan_size(const lu_batch_plan_t* p) { return p->batch; }
 const int32_t* batch_plan_dev_n(const lu_batch_plan_t* p) { return p->d_n; }
 const int32_t* batch_plan_dev_order(const lu_batch_plan_t* p) { return p->d_order; }
+const int32_t* batch_plan_upto(const lu_batch_plan_t* p) { return p->h_upto.data(); }
 int batch_plan_nmax(const lu_batch_plan_t* p) { return p->nmax; }
 }  // namespace lub
 
@@ -731,6 +733,9 @@ LU_API lu_status lu_batch_plan_create(const lu_opts* opts, int64_t batch,
   std::stable_sort(p->h_order.begin(), p->h_order.end(),
                    [&](int32_t x, int32_t y) { return p->h_n[x] > p->h_n[y]; });
   p->nmax = batch > 0 ? p->h_n[p->h_order[0]] : 1;
+  p->h_upto.assign(LU_BATCH_MAX_N + 1, 0);
+  for (int64_t i = 0; i < batch; ++i) ++p->h_upto[h_n[i]];
+  std::partial_sum(p->h_upto.begin(), p->h_upto.end(), p->h_upto.begin());
   lu_status s = LU_SUCCESS;
   if (cudaGetDevice(&p->device) != cudaSuccess) s = LU_ERR_NO_DEVICE;
   const size_t nb = std::max<int64_t>(batch, 1);

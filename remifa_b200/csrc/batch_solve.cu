@@ -1,9 +1,13 @@
 // Batched solves and adjoint for the factors a batch plan produced (new; the
 // reference has neither a batch nor a derivative).
 //
-// One CTA of eight warps per (matrix, group of up to NR right-hand sides); b,
-// x and the residual of the group live in shared memory (fp64), the fp32
-// factors and matrices are read from global memory / L2.
+// Two kernels share a batch, by size (launch_batch_solve): batch_solve_kernel
+// takes the larger matrices, batch_solve_warp_kernel small ones in great number.
+// Both keep b, x and the residual in shared memory (fp64) and read the fp32
+// factors and matrices from global memory / L2.
+//
+// batch_solve_kernel: one CTA of eight warps per (matrix, group of up to NR
+// right-hand sides).
 //   * The 32 x 32 diagonal blocks of L and U are inverted once per item, in
 //     fp64, by substitution (one warp per block, lane j column j), and kept
 //     packed L^-1 \ U^-1 in shared memory; all 1 + refine_iters solves use
@@ -15,11 +19,15 @@
 //     down the rows, one shuffle tree per column.  Both read the factor's
 //     columns coalesced.  While one warp multiplies by Dinv_t the others
 //     already sum block t+1's row over the blocks before t.
+// batch_solve_warp_kernel: one warp per (matrix, right-hand side), down the
+// triangles column by column with no barrier; it fills the chip with matrices
+// where a CTA per matrix would mostly wait (4,000 of n = 40, one right-hand side:
+// 38 us, 129 with the CTA kernel).
 // With the original fp32 matrices given, refine_iters rounds of FP64
 // refinement follow: r = b - op(A) x in fp64, x += op(LU)^-1 r.  Every sum has
 // a fixed order, so results do not depend on scheduling.
 //
-// What bounds it: the chain of dependent block steps (2 (1 + iters) n / 32 of
+// What bounds the CTA kernel: the chain of dependent block steps (2 (1 + iters) n / 32 of
 // them, each an L2 latency and the inverse's product), hidden by three CTAs
 // per SM at n <= 256; there the factors of the resident matrices outgrow L2,
 // so every round reads them from DRAM again (2 TB/s).  The fp32 -> fp64
@@ -42,7 +50,8 @@ namespace lub {
 // plan accessors (batch.cu)
 int64_t batch_plan_size(const lu_batch_plan_t* p);
 const int32_t* batch_plan_dev_n(const lu_batch_plan_t* p);
-const int32_t* batch_plan_dev_order(const lu_batch_plan_t* p);
+const int32_t* batch_plan_dev_order(const lu_batch_plan_t* p);  // by decreasing size
+const int32_t* batch_plan_upto(const lu_batch_plan_t* p);  // [n]: matrices of size <= n
 int batch_plan_nmax(const lu_batch_plan_t* p);
 
 namespace {
@@ -377,13 +386,21 @@ struct SolveArgs {
   int64_t batch;
   int nrhs;
   int iters;
-  const int32_t* order;     // matrices by decreasing size
+  const int32_t* order;     // this launch's matrices (batch of them)
 };
+
+// The launches of one call share a stream and take disjoint matrices: each lets
+// the next one start beside it, and completes only after the one in front.
+__device__ __forceinline__ void launch_begin() { dependents_launch(); }
+__device__ __forceinline__ void launch_end() {
+  if (blockIdx.x == 0) dependency_wait();
+}
 
 template <bool TRANS, int NR>
 __global__ void __launch_bounds__(kT, 3)
 batch_solve_kernel(SolveArgs s) {
   extern __shared__ __align__(16) double sh[];
+  launch_begin();
   const int groups = (s.nrhs + NR - 1) / NR;
   const int64_t item = blockIdx.x;
   const int64_t m = s.order[item / groups];
@@ -422,12 +439,162 @@ batch_solve_kernel(SolveArgs s) {
     const int c = e / np, i = e - c * np;
     if (i < n) xg[i + (int64_t)c * n] = xb[e];
   }
+  launch_end();
+}
+
+// ---- one warp per (matrix, right-hand side) --------------------------------
+namespace warp {
+
+constexpr int kWarpsPerCta = 4;
+
+// x (shared, fp64, length n) <- L^-1 x, L unit lower (fp32, column-major).
+__device__ __forceinline__ void lower_solve(const float* __restrict__ F, int64_t ld,
+                                            int n, double* x) {
+  const int lane = threadIdx.x & 31;
+  for (int j = 0; j < n - 1; ++j) {
+    __syncwarp();
+    const double xj = x[j];
+    const float* col = F + (int64_t)j * ld;
+    for (int i = j + 1 + lane; i < n; i += 32) x[i] = fma(-(double)col[i], xj, x[i]);
+  }
+  __syncwarp();
+}
+
+// x <- U^-1 x, U upper with its diagonal (column form, bottom up).
+__device__ __forceinline__ void upper_solve(const float* __restrict__ F, int64_t ld,
+                                            int n, double* x) {
+  const int lane = threadIdx.x & 31;
+  for (int j = n - 1; j >= 0; --j) {
+    __syncwarp();
+    const float* col = F + (int64_t)j * ld;
+    const double xj = x[j] / (double)col[j];
+    __syncwarp();
+    if (lane == 0) x[j] = xj;
+    for (int i = lane; i < j; i += 32) x[i] = fma(-(double)col[i], xj, x[i]);
+  }
+  __syncwarp();
+}
+
+__device__ __forceinline__ double warp_sum(double v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// x <- U^-T x (dot form, top down: x_j = (x_j - U[0:j, j] . x[0:j]) / U_jj).
+__device__ __forceinline__ void upper_t_solve(const float* __restrict__ F, int64_t ld,
+                                              int n, double* x) {
+  const int lane = threadIdx.x & 31;
+  for (int j = 0; j < n; ++j) {
+    const float* col = F + (int64_t)j * ld;
+    double p = 0.0;
+    for (int i = lane; i < j; i += 32) p = fma((double)col[i], x[i], p);
+    p = warp_sum(p);
+    if (lane == 0) x[j] = (x[j] - p) / (double)col[j];
+    __syncwarp();
+  }
+}
+
+// x <- L^-T x (dot form, bottom up: x_j = x_j - L[j+1:n, j] . x[j+1:n]).
+__device__ __forceinline__ void lower_t_solve(const float* __restrict__ F, int64_t ld,
+                                              int n, double* x) {
+  const int lane = threadIdx.x & 31;
+  for (int j = n - 2; j >= 0; --j) {
+    const float* col = F + (int64_t)j * ld;
+    double p = 0.0;
+    for (int i = j + 1 + lane; i < n; i += 32) p = fma((double)col[i], x[i], p);
+    p = warp_sum(p);
+    if (lane == 0) x[j] = x[j] - p;
+    __syncwarp();
+  }
+}
+
+template <bool TRANS>
+__device__ __forceinline__ void solve(const float* F, int64_t ld, int n, double* x) {
+  if (!TRANS) {
+    lower_solve(F, ld, n, x);
+    upper_solve(F, ld, n, x);
+  } else {
+    upper_t_solve(F, ld, n, x);
+    lower_t_solve(F, ld, n, x);
+  }
+}
+
+// r = b - op(A) x (A fp32, fp64 arithmetic).
+template <bool TRANS>
+__device__ __forceinline__ void residual(const float* __restrict__ A, int64_t ld, int n,
+                                         const double* b, const double* x, double* r) {
+  const int lane = threadIdx.x & 31;
+  if (!TRANS) {
+    for (int i = lane; i < n; i += 32) r[i] = b[i];
+    for (int j = 0; j < n; ++j) {
+      __syncwarp();
+      const double xj = x[j];
+      const float* col = A + (int64_t)j * ld;
+      for (int i = lane; i < n; i += 32) r[i] = fma(-(double)col[i], xj, r[i]);
+    }
+  } else {
+    for (int j = 0; j < n; ++j) {
+      const float* col = A + (int64_t)j * ld;
+      double p = 0.0;
+      for (int i = lane; i < n; i += 32) p = fma((double)col[i], x[i], p);
+      p = warp_sum(p);
+      if (lane == 0) r[j] = b[j] - p;
+    }
+  }
+  __syncwarp();
+}
+
+}  // namespace warp
+
+// nmax: the largest of this launch's matrices.
+template <bool TRANS>
+__global__ void __launch_bounds__(32 * warp::kWarpsPerCta)
+batch_solve_warp_kernel(SolveArgs s, int nmax) {
+  extern __shared__ __align__(16) double sh[];
+  launch_begin();
+  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  double* xb = sh + (size_t)wid * 3 * nmax;
+  double* bb = xb + nmax;
+  double* rb = bb + nmax;
+  const int64_t items = s.batch * s.nrhs;
+  for (int64_t it = (int64_t)blockIdx.x * warp::kWarpsPerCta + wid; it < items;
+       it += (int64_t)gridDim.x * warp::kWarpsPerCta) {
+    const int64_t q = it / s.nrhs;
+    const int c = (int)(it - q * s.nrhs);
+    const int64_t m = s.order[q];
+    const int n = s.n[m];
+    const float* F = s.lu[m];
+    const int64_t ldf = s.ldlu ? s.ldlu[m] : n;
+    double* xg = s.x[m] + (int64_t)c * n;
+    for (int i = lane; i < n; i += 32) {
+      xb[i] = xg[i];
+      bb[i] = xg[i];
+    }
+    __syncwarp();
+    warp::solve<TRANS>(F, ldf, n, xb);
+    if (s.a) {
+      const float* A = s.a[m];
+      const int64_t lda = s.lda ? s.lda[m] : n;
+      for (int k = 0; k < s.iters; ++k) {
+        warp::residual<TRANS>(A, lda, n, bb, xb, rb);
+        warp::solve<TRANS>(F, ldf, n, rb);
+        for (int i = lane; i < n; i += 32) xb[i] += rb[i];
+        __syncwarp();
+      }
+    }
+    for (int i = lane; i < n; i += 32) xg[i] = xb[i];
+    __syncwarp();
+  }
+  launch_end();
 }
 
 // dA_m[i, j] = -sum_r dB_m[i, r] X_m[j, r], one CTA per matrix (largest
 // first): warps take columns j, lanes rows i, dB and X through L1; the writes
-// of dA bound it (1,024 matrices of 64..256: 38 us = 3.0 TB/s; 147 us with an
-// index division per element).
+// of dA bound it (1,024 matrices of 64..256: 38 us = 3.0 TB/s; 147 us with a
+// thread and an index division per element, which is the faster one below 64
+// rows, where it keeps all threads busy: 16000 of n = 16 20 us, 35 by columns; n
+// = 48 112 and 119, n = 64 190 and 138).
 __global__ void __launch_bounds__(kT)
 batch_outer_kernel(const double* const* __restrict__ db, const double* const* __restrict__ x,
                    float* const* __restrict__ da, const int32_t* __restrict__ ldda,
@@ -439,6 +606,16 @@ batch_outer_kernel(const double* const* __restrict__ db, const double* const* __
   const double* __restrict__ G = db[m];
   const double* __restrict__ X = x[m];
   float* __restrict__ D = da[m];
+  if (n < 64) {
+    for (int e = threadIdx.x; e < n * n; e += kT) {
+      const int j = e / n, i = e - j * n;
+      double acc = 0.0;
+      for (int r = 0; r < nrhs; ++r)
+        acc = fma(G[i + (int64_t)r * n], X[j + (int64_t)r * n], acc);
+      D[i + j * ld] = (float)(-acc);
+    }
+    return;
+  }
   constexpr int CW = 4;  // columns of a warp per pass over the rows
   for (int j0 = CW * warp; j0 < n; j0 += CW * kWarps) {
     for (int i = lane; i < n; i += 32) {
@@ -456,24 +633,99 @@ batch_outer_kernel(const double* const* __restrict__ db, const double* const* __
   }
 }
 
-template <bool TRANS, int NR>
-lu_status launch_solve(cudaStream_t st, const SolveArgs& s, int nmax) {
-  const size_t smem = smem_doubles(nmax, NR) * sizeof(double);
-  const int64_t items = s.batch * ((s.nrhs + NR - 1) / NR);
-  if (items > 0x7fffffffll) return LU_ERR_INVALID_ARG;
-  LUB_CUDA_TRY(set_smem_limit((const void*)batch_solve_kernel<TRANS, NR>, smem));
-  batch_solve_kernel<TRANS, NR><<<(unsigned)items, kT, smem, st>>>(s);
+// One launch of a call; `behind`: another launch of the call is in front of it.
+template <typename... P, typename... A>
+lu_status launch_part(bool behind, void (*kernel)(P...), int64_t grid, int threads, size_t smem,
+                      cudaStream_t st, A... args) {
+  LUB_CUDA_TRY(set_smem_limit((const void*)kernel, smem));
+  if (behind) {
+    LUB_CUDA_TRY(launch_dependent(kernel, (unsigned)grid, threads, smem, st, args...));
+  } else {
+    kernel<<<(unsigned)grid, threads, smem, st>>>(args...);
+  }
   LUB_LAUNCH_CHECK();
   return LU_SUCCESS;
+}
+
+// CTAs of batch_solve_kernel an SM holds: its shared memory, at most three.
+int ctas_per_sm(int n, int nr) {
+  return (int)std::min<size_t>(3, 233472 / (smem_doubles(n, nr) * sizeof(double) + 1024));
+}
+
+// The size up to which matrices go to the warp kernel: where the time it needs --
+// the longer of one warp's chain and the sum over all -- stays below what the same
+// matrices cost as CTAs, three to an SM (a fifth less while they stay in L2).  In
+// us, fitted on B200 to uniform batches of 64 .. 16000 matrices of 16 .. 192 rows, 1
+// .. 8 right-hand sides and 0 .. 4 rounds, where 98 % of the cases come within 5 % of the
+// better kernel (the CTA kernel alone takes up to 7 times the warp kernel's time,
+// 16000 of n = 16; the warp kernel alone up to 25 times the other's, 64 of n =
+// 192).
+int warp_limit(const int32_t* upto, int nmax, int nrhs, int nr, int iters, bool trans) {
+  const double block = nr < 4 ? 7.7 : 8.7;
+  const double round = trans ? (nr < 4 ? 3.0 : 8.5) : (nr < 4 ? 2.5 : 4.1);
+  const double slots = 3.0 * sm_count() / ((nrhs + nr - 1) / nr);
+  const double passes = 1.0 + (trans ? 1.45 : 1.27) * iters;
+  double cta = 0.0, sum = 0.0, bytes = 0.0, best = 0.0;
+  int limit = 0;
+  for (int n = 1; n <= std::min(nmax, 160); ++n) {
+    const double c = upto[n] - upto[n - 1], n2 = (double)n * n;
+    if (c == 0.0) continue;
+    const int nb = (n + BS - 1) / BS;
+    cta += c / slots * (12.6 + nb * (block + round * iters));
+    bytes += c * n2 * (iters > 0 ? 8.0 : 4.0);
+    sum += c * nrhs * passes * 1e-3 * (trans ? 0.19 * n + 0.0027 * n2 : 0.052 * n + 0.0045 * n2);
+    const double chain = passes * (trans ? 0.84 * n + 0.0045 * n2 : 0.37 * n + 0.0105 * n2);
+    const double gain = (bytes < 64e6 ? 0.8 : 1.0) * cta - std::max(chain, sum);
+    if (gain > best) {
+      best = gain;
+      limit = n;
+    }
+  }
+  return limit;
+}
+
+template <bool TRANS, int NR>
+lu_status launch_sizes(cudaStream_t st, SolveArgs s, const int32_t* upto, int nmax) {
+  const int32_t* order = s.order;
+  const int64_t batch = s.batch, groups = (s.nrhs + NR - 1) / NR;
+  const int limit = warp_limit(upto, nmax, s.nrhs, NR, s.iters, TRANS);
+  const int64_t big = batch - upto[limit];   // the first ones of `order`
+  if (big * groups > 0x7fffffffll) return LU_ERR_INVALID_ARG;
+  int64_t at = 0;
+  int top = nmax;                            // the largest size from `at` on
+  while (at < big) {
+    // matrices that fit more CTAs on an SM get a launch of their own once they
+    // fill it (1,000 of 64 .. 200 rows and one of 300, five right-hand sides:
+    // 504 us in one launch)
+    const int fit = ctas_per_sm(top, NR);
+    int64_t to = big;
+    int n = top;
+    while (n > limit && ctas_per_sm(n, NR) == fit) --n;
+    if (n > limit && (upto[n] - upto[limit]) * groups > (int64_t)sm_count() * (fit + 1))
+      to = batch - upto[n];
+    s.order = order + at;
+    s.batch = to - at;
+    LUB_TRY(launch_part(at > 0, batch_solve_kernel<TRANS, NR>, s.batch * groups, kT,
+                        smem_doubles(top, NR) * sizeof(double), st, s));
+    at = to;
+    for (top = n; top > limit && upto[top] == upto[top - 1]; --top) {}
+  }
+  if (big == batch) return LU_SUCCESS;
+  s.order = order + big;
+  s.batch = batch - big;
+  const int64_t ctas = std::min<int64_t>(
+      (s.batch * s.nrhs + warp::kWarpsPerCta - 1) / warp::kWarpsPerCta, (int64_t)sm_count() * 16);
+  return launch_part(big > 0, batch_solve_warp_kernel<TRANS>, ctas, 32 * warp::kWarpsPerCta,
+                     (size_t)warp::kWarpsPerCta * 3 * limit * sizeof(double), st, s, limit);
 }
 
 // Right-hand sides per CTA: a second and a fourth column reuse the factor
 // entries already loaded and the inverted blocks.
 template <bool TRANS>
-lu_status launch_batch_solve(cudaStream_t st, const SolveArgs& s, int nmax) {
-  if (s.nrhs == 1) return launch_solve<TRANS, 1>(st, s, nmax);
-  if (s.nrhs == 2) return launch_solve<TRANS, 2>(st, s, nmax);
-  return launch_solve<TRANS, 4>(st, s, nmax);
+lu_status launch_batch_solve(cudaStream_t st, const SolveArgs& s, const int32_t* upto, int nmax) {
+  if (s.nrhs == 1) return launch_sizes<TRANS, 1>(st, s, upto, nmax);
+  if (s.nrhs == 2) return launch_sizes<TRANS, 2>(st, s, upto, nmax);
+  return launch_sizes<TRANS, 4>(st, s, upto, nmax);
 }
 
 }  // namespace
@@ -504,9 +756,10 @@ LU_API lu_status lu_batch_solve_c(lu_batch_plan plan, lu_stream_t stream,
   s.nrhs = nrhs;
   s.iters = d_a ? refine_iters : 0;
   s.order = batch_plan_dev_order(plan);
+  const int32_t* upto = batch_plan_upto(plan);
   const int nmax = batch_plan_nmax(plan);
-  return trans ? launch_batch_solve<true>((cudaStream_t)stream, s, nmax)
-               : launch_batch_solve<false>((cudaStream_t)stream, s, nmax);
+  return trans ? launch_batch_solve<true>((cudaStream_t)stream, s, upto, nmax)
+               : launch_batch_solve<false>((cudaStream_t)stream, s, upto, nmax);
 }
 
 LU_API lu_status lu_batch_adjoint_c(lu_batch_plan plan, lu_stream_t stream,
