@@ -88,14 +88,24 @@ class MatrixBatch:
         if (data.dtype != torch.float32 or data.dim() != 1 or not data.is_contiguous()
                 or data.numel() < int(self.offsets[-1]) or data.device != self.data.device):
             return self.like(data)  # its checks, or another device
+        self._used_here()
         m = object.__new__(MatrixBatch)
         m.__dict__.update(self.__dict__)
         m.data = data
         m.ptrs = self._d_off + data.data_ptr()
         return m
 
+    def _used_here(self) -> None:
+        """The current stream reads the shared device arrays, which may be another
+        stream's: their memory is not handed out again before it has passed here."""
+        if self.data.is_cuda:
+            here = torch.cuda.current_stream(self.data.device)
+            self.d_lda.record_stream(here)   # one storage with d_n
+            self._d_off.record_stream(here)  # one storage with _d_rows
+
     def _rhs_ptrs(self, data: torch.Tensor, nrhs: int) -> torch.Tensor:
         """RhsBatch(self.sizes, nrhs, data=data).ptrs, formed as in _over."""
+        self._used_here()
         return torch.add(self._d_rows * (8 * nrhs), data.data_ptr())
 
     @property
