@@ -88,7 +88,6 @@ class MatrixBatch:
         if (data.dtype != torch.float32 or data.dim() != 1 or not data.is_contiguous()
                 or data.numel() < int(self.offsets[-1]) or data.device != self.data.device):
             return self.like(data)  # its checks, or another device
-        self._used_here()
         m = object.__new__(MatrixBatch)
         m.__dict__.update(self.__dict__)
         m.data = data
@@ -97,7 +96,8 @@ class MatrixBatch:
 
     def _used_here(self) -> None:
         """The current stream reads the shared device arrays, which may be another
-        stream's: their memory is not handed out again before it has passed here."""
+        stream's: their memory is not handed out again before it has passed here.
+        Once per pass that makes views (about 4 us of host time)."""
         if self.data.is_cuda:
             here = torch.cuda.current_stream(self.data.device)
             self.d_lda.record_stream(here)   # one storage with d_n
@@ -105,7 +105,6 @@ class MatrixBatch:
 
     def _rhs_ptrs(self, data: torch.Tensor, nrhs: int) -> torch.Tensor:
         """RhsBatch(self.sizes, nrhs, data=data).ptrs, formed as in _over."""
-        self._used_here()
         return torch.add(self._d_rows * (8 * nrhs), data.data_ptr())
 
     @property
@@ -305,6 +304,7 @@ class BatchedLUSolve(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, a_flat, b_flat, layout, plan, nrhs, refine_iters):
+        layout._used_here()
         a = layout._over(a_flat.detach().contiguous())
         lu = layout._over(a.data.clone())
         info = plan(lu)
@@ -322,6 +322,7 @@ class BatchedLUSolve(torch.autograd.Function):
     def backward(ctx, gx):
         a_d, lu_d, x_d = ctx.saved_tensors
         lay = ctx.layout
+        lay._used_here()
         a, lu = lay._over(a_d), lay._over(lu_d)
         x = RhsBatch._over(lay, ctx.nrhs, x_d)
         g = RhsBatch._over(lay, ctx.nrhs, gx.to(torch.float64).contiguous().clone())

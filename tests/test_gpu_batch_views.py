@@ -4,7 +4,8 @@ import numpy as np
 import pytest
 import torch
 
-from remifa_b200.batch import MatrixBatch, RhsBatch
+import remifa_b200 as rb
+from remifa_b200.batch import BatchPlan, MatrixBatch, RhsBatch, batched_lu_solve
 
 pytestmark = pytest.mark.gpu
 
@@ -29,28 +30,30 @@ def test_pointers(built, sizes, align):
         lay._over(data[:int(lay.offsets[-1]) - 1])
 
 
-@pytest.mark.parametrize("view", ["matrices", "right_hand_sides"])
-def test_shared_arrays_outlive_their_layout_on_another_stream(built, view):
-    """A layout dropped while another stream still reads its device arrays: the
-    arrays' memory is not handed out to its own stream meanwhile."""
+def test_shared_arrays_outlive_their_layout_on_another_stream(built):
+    """A layout dropped while another stream still has to read its device arrays:
+    their memory is not handed out to its own stream meanwhile."""
     sizes = np.full(1500, 4, np.int32)
-    lay = MatrixBatch(sizes)
-    mem = [t.untyped_storage() for t in (lay.d_lda, lay._d_off)]
-    used = {m.data_ptr(): m.nbytes() for m in mem}
-    mem.clear()
+    lay = MatrixBatch(sizes).generate(seed=1)
+    plan = BatchPlan(sizes, outer=rb.FP32)
+    shared = {t.untyped_storage().data_ptr(): t.untyped_storage().nbytes()
+              for t in (lay.d_lda, lay._d_off)}
     side = torch.cuda.Stream()
     side.wait_stream(torch.cuda.current_stream())
     with torch.cuda.stream(side):
-        data = torch.zeros(int(lay.offsets[-1]), device="cuda")
-        x = torch.zeros(int(sizes.sum()), dtype=torch.float64, device="cuda")
-        torch.cuda._sleep(100_000_000)
-        got = lay._over(data) if view == "matrices" else RhsBatch._over(lay, 1, x)
-    shared = [lay._d_off.untyped_storage().data_ptr()]
-    if view == "matrices":
-        shared.append(lay.d_lda.untyped_storage().data_ptr())
-    del got, lay
-    new = [torch.empty(n, dtype=torch.uint8, device="cuda") for n in used.values()
+        a = lay.data.clone().requires_grad_(True)
+        b = torch.ones(int(sizes.sum()), dtype=torch.float64, device="cuda", requires_grad=True)
+        # once before, so that nothing below loads a kernel or takes new memory
+        warm = batched_lu_solve(a, b, MatrixBatch(sizes), plan)
+        torch.autograd.grad(warm, (a, b), torch.ones_like(warm))
+        del warm
+        x = batched_lu_solve(a, b, lay, plan)
+        torch.cuda._sleep(200_000_000)
+        grads = torch.autograd.grad(x, (a, b), torch.ones_like(x))
+    del x, lay
+    new = [torch.empty(n, dtype=torch.uint8, device="cuda") for n in shared.values()
            for _ in range(8)]
     assert not side.query()
     assert not {t.data_ptr() for t in new} & set(shared)
     side.synchronize()
+    assert all(bool(torch.isfinite(g).all()) for g in grads)
