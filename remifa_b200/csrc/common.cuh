@@ -7,6 +7,7 @@
 #include <cuda_fp8.h>
 #include <cstdint>
 #include <cstdio>
+#include <utility>
 
 #include "lu_b200.h"
 
@@ -169,6 +170,16 @@ __device__ __forceinline__ bool factor_tile8_fast(float* T, int LD, float* inv) 
 __device__ __forceinline__ void dependency_wait() { cudaGridDependencySynchronize(); }
 __device__ __forceinline__ void dependents_launch() { cudaTriggerProgrammaticLaunchCompletion(); }
 
+// A launch that fails is reported by its return value alone: the runtime's last
+// error is cleared, so that no later launch check, ours or the program's, sees it.
+template <typename... P, typename... A>
+inline cudaError_t launch_config(const cudaLaunchConfig_t& cfg, void (*kernel)(P...),
+                                 A&&... args) {
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+  if (e != cudaSuccess) (void)cudaGetLastError();
+  return e;
+}
+
 template <typename... P, typename... A>
 inline cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
                                     cudaStream_t st, A&&... args) {
@@ -182,7 +193,7 @@ inline cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block,
   cfg.stream = st;
   cfg.attrs = &at;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+  return launch_config(cfg, kernel, std::forward<A>(args)...);
 }
 
 // Record the 1-based global index of a zero / non-finite pivot.

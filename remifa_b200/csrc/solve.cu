@@ -1073,7 +1073,7 @@ lu_status launch_one(cudaStream_t st, const Args& a) {
     at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = 2;
-    LUB_CUDA_TRY(cudaLaunchKernelEx(&cfg, fn, a));
+    LUB_CUDA_TRY(launch_config(cfg, fn, a));
   } else {
     smem = mma_smem_bytes();
     fn = trsv_mma_kernel<TRANS, V16>;
