@@ -184,8 +184,8 @@ __device__ __forceinline__ double reduce4(const double (&a)[4]) {
 // The warp's share of rows [r0, r0 + 32) of op(F) times x over whole blocks of
 // 32 columns: not transposed, lane = row, columns 4 warp .. 4 warp + 3 of each
 // block; transposed, rows 4 warp .. 4 warp + 3 of the row block (columns of
-// F), lanes over the block's 32.  Rows and columns past n read the last valid
-// one instead: x is zero there, and sums of rows past n are dropped.
+// F), lanes over the block's 32.  Rows past n read the last valid one instead
+// (their sums are dropped); columns past n are zero, as x is there.
 template <bool TRANS, int NR>
 struct Partial {
   static constexpr int NA = TRANS ? 4 : 1;
@@ -221,8 +221,7 @@ struct Partial {
 #pragma unroll
       for (int c = 0; c < NR; ++c) acc[q][c] = 0.0;
   }
-  // The warp's entries of block q0: of a whole block, of any (the last valid
-  // row / column in place of those past n).
+  // The warp's entries of block q0: of a whole block, of any.
   __device__ __forceinline__ void fetch_whole(float (&v)[4], int64_t ld, int q0) const {
     const int64_t at = TRANS ? (int64_t)(q0 * BS) : row + q0 * (BS * ld);
 #pragma unroll
@@ -232,10 +231,18 @@ struct Partial {
     if ((q0 + 1) * BS <= n) return fetch_whole(v, ld, q0);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t at = TRANS ? (int64_t)(q0 * BS) : row + q0 * (BS * ld);
+    const int left = n - q0 * BS - (TRANS ? lane : 4 * warp);
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-      const int over = max(0, q0 * BS + (TRANS ? lane : 4 * warp + q) - (n - 1));
-      v[q] = p[q][at - over * (TRANS ? 1 : ld)];
+      if (TRANS && NR == 1) {
+        // loaded and dropped: 440 us, 459 with the load left out (1,024 matrices of
+        // 64..256; the other instances are the faster ones without it)
+        const float y = p[q][at + min(0, left - 1)];
+        v[q] = left > 0 ? y : 0.0f;
+      } else {
+        v[q] = 0.0f;
+        if (left > (TRANS ? 0 : q)) v[q] = p[q][at];
+      }
     }
   }
   // block q0's entries v times x

@@ -877,25 +877,38 @@ trsv_mma_kernel(Args a) {
   cp_commit();
 
   // This warp's share of tile q: entry [m][s] is row 8 m + lr and column kk(s).
-  // Rows and columns past the matrix repeat the last one (their sums are
-  // dropped, or meet zeros of x).
+  // Rows past the matrix repeat the last one (their sums are dropped); only the
+  // first tile of a backward solve has columns past it.
   auto kk = [&](int s) { return 8 * warp + (TRANS ? 2 * lk + s : 4 * s + lk); };
   auto load_a = [&](int q, float (&v)[8][2]) {
     const int64_t k0 = tile_k0(q);
-    const int kw = tile_kw(q);
 #pragma unroll
     for (int m = 0; m < 8; ++m) {
       const int64_t r = r0 + (8 * m + lr < rw ? 8 * m + lr : rw - 1);
-      if (TRANS && V16 && kw == BS) {
+      if (TRANS && V16) {
         const float2 y = *reinterpret_cast<const float2*>(a.lu + k0 + kk(0) + r * a.ld);
         v[m][0] = y.x;
         v[m][1] = y.y;
       } else {
 #pragma unroll
-        for (int s = 0; s < 2; ++s) {
-          const int64_t k = k0 + (kk(s) < kw ? kk(s) : kw - 1);
-          v[m][s] = TRANS ? a.lu[k + r * a.ld] : a.lu[r + k * a.ld];
-        }
+        for (int s = 0; s < 2; ++s)
+          v[m][s] = TRANS ? a.lu[k0 + kk(s) + r * a.ld] : a.lu[r + (k0 + kk(s)) * a.ld];
+      }
+    }
+  };
+  // the first tile, columns past the matrix zero: they meet zeros of x, whose
+  // products with an infinity would not be
+  auto load_first = [&](float (&v)[8][2]) {
+    const int64_t k0 = tile_k0(0);
+    const int kw = tile_kw(0);
+    if (kw == BS) return load_a(0, v);
+#pragma unroll
+    for (int m = 0; m < 8; ++m) {
+      const int64_t r = r0 + (8 * m + lr < rw ? 8 * m + lr : rw - 1);
+#pragma unroll
+      for (int s = 0; s < 2; ++s) {
+        const int64_t k = k0 + kk(s);
+        v[m][s] = kk(s) < kw ? (TRANS ? a.lu[k + r * a.ld] : a.lu[r + k * a.ld]) : 0.0f;
       }
     }
   };
@@ -928,7 +941,7 @@ trsv_mma_kernel(Args a) {
     }
   };
   if (!a.early) fetch_inputs();
-  if (nbulk > 0) load_a(0, cur);
+  if (nbulk > 0) load_first(cur);
   cp_wait<0>();
   __syncthreads();
   invert_diag<TRANS, DS>(Dsrc, Dinv, rdiag, rw, fwd, a.unit != 0);
