@@ -58,24 +58,20 @@ int sm_count() {
 }
 
 cudaError_t set_smem_limit(const void* func, size_t bytes) {
-  // The attribute is per (function, device); remember the largest value set.
+  // The attribute is per (function, device); remember the largest value set.  Set
+  // under the lock: a thread that needs less must not lower what another thread
+  // has just set for its launch.
   static std::unordered_map<uint64_t, size_t> done;
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
-  const uint64_t key = ((uint64_t)(uintptr_t)func) ^ ((uint64_t)dev << 56);
-  {
-    std::lock_guard<std::mutex> lk(g_mu);
-    auto it = done.find(key);
-    if (it != done.end() && it->second >= bytes) return cudaSuccess;
-  }
   if (bytes <= 48 * 1024) return cudaSuccess;
-  e = cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)bytes);
-  if (e == cudaSuccess) {
-    std::lock_guard<std::mutex> lk(g_mu);
-    done[key] = bytes;
-  }
+  const uint64_t key = ((uint64_t)(uintptr_t)func) ^ ((uint64_t)dev << 56);
+  std::lock_guard<std::mutex> lk(g_mu);
+  size_t& limit = done[key];
+  if (limit >= bytes) return cudaSuccess;
+  e = cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (e == cudaSuccess) limit = bytes;
   return e;
 }
 
