@@ -453,6 +453,15 @@ LU_API lu_status lu_selftest_wait_solve_c(lu_stream_t stream, unsigned long long
                                           double* d_x, void* d_scratch, size_t bytes,
                                           unsigned* d_expired);
 
+/* One triangular solve op(T) X = X (T: the unit lower part of d_lu, or with upper
+ * = 1 the upper one; trans = 1: transposed; 1 .. 4 columns, fp64, leading dimension
+ * ldx) without thread-block clusters, the way it runs where none of 16 fit.
+ * d_scratch: device, 256 + 8 n nrhs bytes rounded up to a multiple of 256. */
+LU_API lu_status lu_selftest_solve_alone_c(lu_stream_t stream, int64_t n, int64_t nrhs,
+                                           const float* d_lu, int64_t ldlu, double* d_x,
+                                           int64_t ldx, int upper, int trans, void* d_scratch,
+                                           size_t bytes);
+
 /* One block row of the host entry's left-looking chunk catch-up, for tests
  * and measurement (no reference counterpart; for one block row it stands
  * for the U-panel solves of src/lu_nopiv_inner_rl.hxx:155-190 that the

@@ -142,6 +142,8 @@ SIGNATURES = {
     "lu_selfcheck_rcp_c": (_int, [_vp, _vp]),
     "lu_selftest_wait_update_c": (_int, [_vp, ctypes.c_longlong, _int, _vp, ctypes.c_size_t,
                                          _vp]),
+    "lu_selftest_solve_alone_c": (_int, [_vp, _i64, _i64, _vp, _i64, _vp, _i64, _int, _int, _vp,
+                                         ctypes.c_size_t]),
     "lu_selftest_wait_solve_c": (_int, [_vp, ctypes.c_ulonglong, _i64, _vp, _i64, _vp, _vp,
                                         ctypes.c_size_t, _vp]),
     "lu_catchup_row_step_c": (_int, [_vp, _int, _int, _i64, _i64, _i64, _i64, _vp, _i64, _vp,

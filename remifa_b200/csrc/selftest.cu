@@ -81,4 +81,19 @@ LU_API lu_status lu_selftest_wait_solve_c(lu_stream_t stream, unsigned long long
   return LU_SUCCESS;
 }
 
+LU_API lu_status lu_selftest_solve_alone_c(lu_stream_t stream, int64_t n, int64_t nrhs,
+                                           const float* d_lu, int64_t ldlu, double* d_x,
+                                           int64_t ldx, int upper, int trans, void* d_scratch,
+                                           size_t bytes) {
+  if (n < 1 || nrhs < 1 || nrhs > 4 || ldlu < n || ldx < n || !d_lu || !d_x || !d_scratch ||
+      (upper != 0 && upper != 1) || (trans != 0 && trans != 1))
+    return LU_ERR_INVALID_ARG;
+  if (bytes < trsm_ws_bytes(n, nrhs)) return LU_ERR_WORKSPACE;
+  LUB_TRY(check_device_here());
+  unsigned* sync = static_cast<unsigned*>(d_scratch);
+  double* B = reinterpret_cast<double*>(static_cast<char*>(d_scratch) + trsm_sync_bytes(nrhs));
+  return launch_trsm((cudaStream_t)stream, n, d_lu, ldlu, d_x, ldx, nrhs, upper != 0, trans != 0,
+                     sync, B, 0, -1, true);
+}
+
 }  // extern "C"

@@ -33,7 +33,9 @@
 #include "mma64.cuh"
 #include "solve.cuh"
 
-#include <atomic>
+#include <map>
+#include <mutex>
+#include <tuple>
 
 namespace lub {
 namespace {
@@ -66,6 +68,7 @@ struct Args {
   unsigned long long wait_ns;  // bound of one wait (kWaitNs)
   int withhold;     // self-test of the give-up path only: the row block solved
                     // first (ticket 0) does not publish its solution, -1: none
+  int cluster;      // CTAs of a cluster of the warp kernel: kCluster or 1
 };
 
 __device__ __forceinline__ unsigned long long global_ns() {
@@ -278,7 +281,8 @@ constexpr int S = 3;                   // stages of each warp's tile ring
 // Row blocks solved one after another by the CTAs of one cluster: they hand
 // their solutions over through distributed shared memory (0.6 us a block on
 // B200, against 1.0 through L2 and 1.5 .. 2 from one cluster to the next, which
-// is why 16 rather than the portable 8).
+// is why 16 rather than the portable 8).  Where no cluster of 16 fits (few SMs in a
+// processing cluster of the context), every CTA is its own.
 constexpr int kCluster = 16;
 constexpr int kWarpTile = 8 * BS;      // floats of a warp's share of a tile
 // Marks a solution entry not yet published: a signalling-NaN payload that no
@@ -537,7 +541,7 @@ trsv_kernel(Args a) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (!a.early) dependency_wait();
   dependents_launch();
-  // the cluster's ticket: its kCluster consecutive row blocks of one group
+  // the cluster's ticket: its consecutive row blocks of one group
   const int rank = cluster_rank();
   for (int e = tid; e < kCluster * NR * BS; e += kThreads)
     xin[e] = __longlong_as_double((long long)kPending);
@@ -547,7 +551,7 @@ trsv_kernel(Args a) {
     int tk = 0;
     if (tid == 0) tk = (int)atomicAdd(a.sync, 1u);
     tk = __shfl_sync((1u << kCluster) - 1, tk, 0);
-    st_remote32(ctrl, tid, tk);
+    if (tid < a.cluster) st_remote32(ctrl, tid, tk);
   }
   if (tid == 0) {
     // the store is on its way; bounded like every wait
@@ -558,7 +562,7 @@ trsv_kernel(Args a) {
   }
   __syncthreads();
   const int ticket = ctrl[1];
-  const int base = ticket / a.ngroups * kCluster;     // first block of the cluster
+  const int base = ticket / a.ngroups * a.cluster;    // first block of the cluster
   const int t = base + rank, g = ticket % a.ngroups;
   if (ticket < 0 || t >= a.nblk) {
     cluster_sync();   // as at the end
@@ -785,7 +789,7 @@ trsv_kernel(Args a) {
 #pragma unroll
         for (int h = 0; h < kCluster / 4; ++h) {
           const int to = rank + 1 + (lane & 3) + 4 * h;
-          if (to < kCluster && base + to < a.nblk)
+          if (to < a.cluster && base + to < a.nblk)
             st_remote64(xin + (rank * NR + c) * BS + ri, to, publish_bits(cv[c]));
         }
         if ((lane & 3) == 0) st_publish(a.X + (r0 + ri) + (c0 + c) * a.ldx, cv[c]);
@@ -1053,10 +1057,48 @@ trsv_mma_kernel(Args a) {
 }
 
 // Right-hand sides per CTA: from five on, the matrix kernel's 8; three or four as
-// two groups of two (three, on B200: n = 2000 100 us, 8192 329, 10007 569, against
-// 126, 464 and 636 with the matrix kernel; five would take 100, 482 and 862 in
-// pairs, 132, 498 and 703 with the matrix kernel).
+// two groups of two (three, on B200: n = 2000 100 us, 8192 339, 10007 579, against
+// 126, 464 and 636 with the matrix kernel).  Five in pairs gain little where the
+// three groups fit (n = 2000 100 us against 132, 8192 482 against 498) and lose
+// more where they do not (10007 862 against 703), so n is not in the rule.
 int group_width(int64_t nrhs) { return nrhs >= 5 ? 8 : nrhs >= 2 ? 2 : 1; }
+
+cudaLaunchAttribute cluster_attribute() {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = kCluster;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  return at;
+}
+
+// Whether clusters of kCluster CTAs of fn (a trsv_kernel) can run with this shared
+// memory, asked once per kernel, device and amount (two columns have two).
+bool clusters_fit(const void* fn, size_t smem) {
+  static std::mutex mu;
+  static std::map<std::tuple<const void*, int, size_t>, bool> known;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return false;
+  std::lock_guard<std::mutex> lk(mu);
+  const auto key = std::make_tuple(fn, dev, smem);
+  const auto it = known.find(key);
+  if (it != known.end()) return it->second;
+  cudaLaunchAttribute at = cluster_attribute();
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(kCluster);
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  // clusters of more than 8 CTAs are allowed per kernel
+  int n = 0;
+  if (cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
+          cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&n, fn, &cfg) != cudaSuccess) {
+    (void)cudaGetLastError();
+    n = 0;
+  }
+  return known[key] = n > 0;
+}
 
 template <bool TRANS, int NR, bool V16>
 lu_status launch_one(cudaStream_t st, const Args& a) {
@@ -1068,30 +1110,20 @@ lu_status launch_one(cudaStream_t st, const Args& a) {
     smem = warp_smem_bytes(NR) + (NR == 2 && a.ngroups == 1 ? (size_t)8 * NR * BS * 8 : 0);
     fn = trsv_kernel<TRANS, NR, V16>;
     LUB_CUDA_TRY(set_smem_limit((const void*)fn, smem));
-    // clusters of more than 8 CTAs are allowed per kernel, once per device
-    static std::atomic<uint64_t> allowed{0};
-    int dev = 0;
-    LUB_CUDA_TRY(cudaGetDevice(&dev));
-    const uint64_t bit = 1ull << (dev & 63);
-    if (!(allowed.load() & bit)) {
-      LUB_CUDA_TRY(cudaFuncSetAttribute((const void*)fn,
-                                        cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-      allowed.fetch_or(bit);
-    }
+    Args b = a;
+    if (a.cluster != 1) b.cluster = clusters_fit((const void*)fn, smem) ? kCluster : 1;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(ceil_div(a.nblk, kCluster) * kCluster * a.ngroups));
+    cfg.gridDim = dim3((unsigned)(ceil_div(a.nblk, b.cluster) * b.cluster * a.ngroups));
     cfg.blockDim = dim3(kThreads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute at[2];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = kCluster;
-    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[1].val.programmaticStreamSerializationAllowed = 1;
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1] = cluster_attribute();
     cfg.attrs = at;
-    cfg.numAttrs = 2;
-    LUB_CUDA_TRY(launch_config(cfg, fn, a));
+    cfg.numAttrs = b.cluster > 1 ? 2 : 1;
+    LUB_CUDA_TRY(launch_config(cfg, fn, b));
   } else {
     smem = mma_smem_bytes();
     fn = trsv_mma_kernel<TRANS, V16>;
@@ -1447,7 +1479,7 @@ namespace {
 lu_status launch_pass(cudaStream_t st, int64_t n, const float* lu, int64_t ld, double* X,
                       int64_t ldx, double* B, int64_t ldb, int64_t nrhs, bool upper, bool trans,
                       unsigned* sync, bool mark, bool early, unsigned long long wait_ns,
-                      int withhold) {
+                      int withhold, bool alone = false) {
   const int nr = trsv::group_width(nrhs);
   if (ceil_div(n, trsv::BS) * ceil_div(nrhs, nr) > 0x7fffffffll) return LU_ERR_INVALID_ARG;
   trsv::Args a;
@@ -1469,6 +1501,7 @@ lu_status launch_pass(cudaStream_t st, int64_t n, const float* lu, int64_t ld, d
   a.sync = sync;
   a.wait_ns = wait_ns > 0 ? wait_ns : trsv::kWaitNs;
   a.withhold = withhold;
+  a.cluster = alone ? 1 : trsv::kCluster;
   const bool v16 = ((reinterpret_cast<uintptr_t>(lu) & 15) == 0) && (ld % 4 == 0);
   if (trans)
     return v16 ? trsv::launch_nr<true, true>(st, a, nr) : trsv::launch_nr<true, false>(st, a, nr);
@@ -1488,12 +1521,12 @@ lu_status launch_prepare(cudaStream_t st, int64_t n, int64_t nrhs, double* X, in
 lu_status launch_trsm(cudaStream_t st, int64_t n, const float* lu, int64_t ld,
                       double* X, int64_t ldx, int64_t nrhs, bool upper,
                       bool trans, unsigned* sync, double* B,
-                      unsigned long long wait_ns, int withhold) {
+                      unsigned long long wait_ns, int withhold, bool alone) {
   if (n <= 0 || nrhs <= 0) return LU_SUCCESS;
   if (!sync || !B) return LU_ERR_INVALID_ARG;
   LUB_TRY(launch_prepare(st, n, nrhs, X, ldx, B, sync));
   return launch_pass(st, n, lu, ld, X, ldx, B, n, nrhs, upper, trans, sync, false, false, wait_ns,
-                     withhold);
+                     withhold, alone);
 }
 
 // The first pass takes its right-hand sides from X, leaves X pending and solves
