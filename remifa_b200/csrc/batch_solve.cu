@@ -33,7 +33,7 @@
 // so every round reads them from DRAM again (2 TB/s).  The fp32 -> fp64
 // conversions (one warp instruction per 8 cycles and scheduler) take a
 // seventh of the time, the arithmetic less.  1,024 matrices of 64..256, one
-// right-hand side, 4 refinement rounds on B200: 0.44 ms (transposed 0.43),
+// right-hand side, 4 refinement rounds on B200: 0.42 ms (transposed 0.44),
 // 6.3 ms as one warp per (matrix, right-hand side) walking single columns.
 //
 // The adjoint of X = A^-1 B: dB = A^-T G (the transposed solve above, in
@@ -73,8 +73,11 @@ __host__ __device__ inline size_t smem_doubles(int nmax, int nr) {
 // warp per block.  The 16 x 16 diagonal halves by substitution (half-warp h
 // half h, lane j column j), then the off-diagonal quarters as products:
 // -L22^-1 L21 L11^-1 by the lower half-warp, -U11^-1 U12 U22^-1 by the upper
-// one (half the registers of a 32-row substitution, so three CTAs fit; a
-// rolled form of this code took 25 us more on 1,024 matrices of 64..256).
+// one (half the registers of a 32-row substitution).  This sets the kernel's
+// register need: at the 80 that three CTAs per SM leave, its instances spill 120 to
+// 570 bytes a thread, most of them here; two CTAs at 128 registers took 465 us
+// where three take 430, a rolled form of this code 25 us more (1,024 matrices of
+// 64..256).
 __device__ __forceinline__ void invert_blocks(const float* __restrict__ F, int64_t ld, int n,
                                               int nb, double* S) {
   constexpr int H = BS / 2;

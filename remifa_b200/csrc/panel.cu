@@ -129,7 +129,8 @@ __device__ __noinline__ void factor_tile_thread(float* T, int LD, int tw,
 //
 // The tile warp has an SM sub-partition to itself: the owners are the warps
 // whose index is not a multiple of four (beside the owners its chain of
-// dependent instructions took up to twice as long).
+// dependent instructions took up to twice as long).  The other multiples of four
+// do nothing but keep it so; with their registers the kernel fills an SM.
 constexpr int kOwnerWarps = 16;
 constexpr int kDiagLD = 132;           // leading dimension of CROUT's block
 constexpr int kDiagThreads = 704;      // warps 0 .. 21: the tile warp, 16 owners
@@ -141,7 +142,7 @@ __device__ __forceinline__ void diag_sync() {
 struct DiagSmem {
   float L[2][8 * 128];   // strips: column k of tile t's L rows, row r at [k * 128 + r]
   float U[2][8 * 128];   // row k of its U columns, column c at [k * 128 + c]
-  float next[2][64];     // tile t+2's block after update t-1 (CROUT: its sums)
+  float next[2][64];     // tile t+2's block after update t (CROUT: its sums)
   float tile[64];        // tile t+1, factored
   float inv[8];
 };

@@ -23,11 +23,11 @@
 // Dinv op(T)[t, t-1] while the CTA waits, so the hand-over from block t-1 to
 // block t is, per warp and without a CTA barrier: x_t = Dinv (b -
 // sum_{q<t-1} op(T)[t,q] x_q) - W x_{t-1}.  trsv_kernel does this with FMAs
-// and shuffles for 1 to 4 right-hand sides (groups of 1 or 2), trsv_mma_kernel on the FP64 matrix
-// instruction for groups of 8.  On B200: one right-hand side, n = 10007, L and U
-// 0.278 ms (0.344 without clusters), n = 16384 0.46 (0.58); 64 right-hand
-// sides, n = 8192 0.82 (1.36 with a counter per group and shared-memory
-// tiles).  Bound by the chain of n / 64 hand-overs.
+// and shuffles for 1 to 4 right-hand sides (groups of 1 or 2), trsv_mma_kernel
+// on the FP64 matrix instruction for groups of 8.  On B200: one right-hand side,
+// n = 10007, L and U 0.277 ms (0.344 without clusters), n = 16384 0.46 (0.58); 64
+// right-hand sides, n = 8192 0.80, transposed 0.81 (1.36 with a counter per group
+// and shared-memory tiles).  Bound by the chain of n / 64 hand-overs.
 #include "common.cuh"
 #include "kernels.cuh"
 #include "mma64.cuh"
@@ -271,7 +271,7 @@ __device__ __forceinline__ double row_reduce(double (&v)[8], int lane) {
 }
 
 // ======================================================================
-// Warp kernel (groups of 1 or 2 right-hand sides).  X is marked pending by
+// Warp kernel (1 to 4 right-hand sides, in groups of 1 or 2).  X is marked pending by
 // trsv_prepare_kernel; a solution entry is published by one store and read
 // by relaxed loads at GPU scope, re-read while pending -- the solution is
 // its own flag.
@@ -799,8 +799,6 @@ trsv_kernel(Args a) {
   cluster_sync();
 }
 
-// B <- X and X <- pending, for the rows and columns of the solve; the first
-// thread also clears the ticket counter and the expired-wait count.
 constexpr int kHeader = 4;   // words of a pass's sync area: ticket, expired waits, spare
 
 // Clears the ticket and expiry words of both passes' sync areas and marks the
@@ -1169,7 +1167,8 @@ residual_partial_kernel(int64_t n, const float* __restrict__ A, int64_t lda,
   if (i >= n) return;
   const float* col = A + i + c0 * lda;
   double acc = 0.0;
-  // few CTAs at the sizes a single solve has: 32 loads in flight per thread
+  // few CTAs at the sizes a single solve has: as many loads in flight per thread as
+  // the kernel's registers hold
 #pragma unroll 32
   for (int k = 0; k < cn; ++k) acc = fma((double)col[k * lda], xs[k], acc);
   P[(int64_t)blockIdx.y * n + i] = acc;
