@@ -70,6 +70,8 @@ class MatrixBatch:
         # byte offsets of the matrices, rows before each matrix
         rows = np.cumsum(self.sizes, dtype=np.int64) - self.sizes
         self._d_off, self._d_rows = torch.from_numpy(np.stack([off[:-1] * 4, rows])).to(device)
+        if data.is_cuda:
+            self._home = torch.cuda.current_stream(device).cuda_stream
 
     def __len__(self) -> int:
         return int(self.sizes.size)
@@ -94,14 +96,22 @@ class MatrixBatch:
         m.ptrs = self._d_off + data.data_ptr()
         return m
 
+    # the stream the device arrays were made on; a copy's are made anew, on its own
+    _home = None
+
+    def __getstate__(self):
+        return {k: v for k, v in self.__dict__.items() if k != "_home"}
+
     def _used_here(self) -> None:
-        """The current stream reads the shared device arrays, which may be another
-        stream's: their memory is not handed out again before it has passed here.
-        Once per pass that makes views (about 4 us of host time)."""
+        """The current stream reads the shared device arrays: where they are another
+        stream's, their memory is not handed out again before it has passed here.
+        Once per pass that makes views (recording costs 10 us of host time, a
+        twentieth of a pass over few small matrices)."""
         if self.data.is_cuda:
             here = torch.cuda.current_stream(self.data.device)
-            self.d_lda.record_stream(here)   # one storage with d_n
-            self._d_off.record_stream(here)  # one storage with _d_rows
+            if here.cuda_stream != self._home:
+                self.d_lda.record_stream(here)   # one storage with d_n
+                self._d_off.record_stream(here)  # one storage with _d_rows
 
     def _rhs_ptrs(self, data: torch.Tensor, nrhs: int) -> torch.Tensor:
         """RhsBatch(self.sizes, nrhs, data=data).ptrs, formed as in _over."""

@@ -1,5 +1,8 @@
 """The device-side pointer arrays batched_lu_solve forms for its buffers equal
 those of the public constructors; its checks stay theirs."""
+import copy
+import pickle
+
 import numpy as np
 import pytest
 import torch
@@ -57,3 +60,14 @@ def test_shared_arrays_outlive_their_layout_on_another_stream(built):
     assert not {t.data_ptr() for t in new} & set(shared)
     side.synchronize()
     assert all(bool(torch.isfinite(g).all()) for g in grads)
+
+
+def test_copies_and_views_know_their_stream(built):
+    """A view shares its layout's arrays and so their stream; a copy's arrays are
+    new, on whatever stream it is made, and are recorded wherever they are used."""
+    lay = MatrixBatch(np.array([3, 5], np.int32))
+    assert lay._home == torch.cuda.current_stream().cuda_stream
+    assert lay._over(torch.zeros_like(lay.data))._home == lay._home
+    for other in (copy.copy(lay), copy.deepcopy(lay), pickle.loads(pickle.dumps(lay))):
+        assert other._home is None
+        assert other.lda.tolist() == lay.lda.tolist()
