@@ -234,15 +234,17 @@ struct Partial {
     if ((q0 + 1) * BS <= n) return fetch_whole(v, ld, q0);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t at = TRANS ? (int64_t)(q0 * BS) : row + q0 * (BS * ld);
-    const int left = n - q0 * BS - (TRANS ? lane : 4 * warp);
+    if (TRANS && NR == 1) {
+      // loaded and dropped: 442 us, 460 with the load left out (1,024 matrices of
+      // 64..256; the other instances are the faster ones without it)
+      const int over = max(0, q0 * BS + lane - (n - 1));
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      if (TRANS && NR == 1) {
-        // loaded and dropped: 440 us, 459 with the load left out (1,024 matrices of
-        // 64..256; the other instances are the faster ones without it)
-        const float y = p[q][at + min(0, left - 1)];
-        v[q] = left > 0 ? y : 0.0f;
-      } else {
+      for (int q = 0; q < 4; ++q) v[q] = p[q][at - over];
+      if (over > 0) v[0] = v[1] = v[2] = v[3] = 0.0f;
+    } else {
+      const int left = n - q0 * BS - (TRANS ? lane : 4 * warp);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
         v[q] = 0.0f;
         if (left > (TRANS ? 0 : q)) v[q] = p[q][at];
       }
