@@ -396,6 +396,7 @@ struct PackTarget {
   const TcWs* w = nullptr;
   int64_t ldk = 0, nb = 0;
   int bf16 = 0;
+  int simt = 0;
   // also the host entry's catch-up copy of the step's L columns (global
   // row r, column c at lp[r * ldl + c]); the step starts at column ofs
   char* lp = nullptr;
@@ -404,6 +405,7 @@ struct PackTarget {
   // offL / offU past the sub-block's edge
   LuPack at(int64_t p0, int wd, int64_t offL, int64_t offU) const {
     LuPack k;
+    k.simt = simt;
     if (!ws) return k;
     k.pa = ws + w->off_a;
     k.pb = ws + w->off_b;
@@ -428,6 +430,7 @@ static bool fused_pack(lu_compute outer) {
 
 static PackTarget pack_target(const Plan& p, char* ws, const TcWs& w) {
   PackTarget t;
+  t.simt = !is_tc(p.outer);
   if (!fused_pack(p.outer)) return t;
   t.ws = ws;
   t.w = &w;

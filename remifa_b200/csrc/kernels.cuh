@@ -26,6 +26,7 @@ struct LuPack {
   void* pa2 = nullptr;
   int64_t ldk2 = 0, row02 = 0;
   int k02 = 0;
+  int simt = 0;   // the trailing updates beside this launch run on the FP32 cores
 };
 
 // L rows (M of them, below) and U columns (N, right) of the w x w factored

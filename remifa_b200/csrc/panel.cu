@@ -14,7 +14,7 @@
 //                        right of it, 32 or 64 rows or columns per CTA (one
 //                        grid for both strips), optionally writing the K-major
 //                        tensor-core operand copies of what it finishes;
-//   lupanel_wide_kernel: the same for large right-looking launches;
+//   lupanel_wide_kernel: the same for large launches beside tensor-core updates;
 //   ref_panel_kernel   : remifa::lu_nopiv_panel<float,8> as a standalone
 //                        entry point (lu_panel_c);
 // each replaying, per element, the reference's exact operation sequence
@@ -414,10 +414,11 @@ diag_factor_kernel(float* __restrict__ a, int64_t lda, int w, int64_t col0,
 // warps left of the current tile drop out.  8 threads per item, 32 items per CTA
 // where that is at most one CTA per SM -- bound by the chain of w / 8 tiles; w =
 // 128 on B200, launches back to back, 256 items of both strips 12.5 us, 16.6 with
-// the items in shared memory -- and 64 in larger left-looking launches, bound by
-// the FMA and shared-memory read rates (fp16 storage, n = 8192: 4.33 ms, 4.48 with
-// lupanel_wide_kernel and the running sums in shared memory).  Larger
-// right-looking launches are lupanel_wide_kernel's.
+// the items in shared memory -- and 64 in larger launches of the left-looking order
+// or beside FP32 updates, bound by the FMA and shared-memory read rates (fp16
+// storage, n = 8192: 4.33 ms, 4.48 with lupanel_wide_kernel and the running sums in
+// shared memory; FP32 with nb = 128, n = 8192 14.4 and 15.6, n = 12000 40.9 and
+// 46.6).  Larger launches beside tensor-core updates are lupanel_wide_kernel's.
 
 // What one CTA works on: its items (row i: a + i, column i: a + i * lda) and
 // the factor values that multiply item value k for position p, both as they
@@ -658,14 +659,14 @@ lupanel_kernel(float* __restrict__ dg, int64_t lda, int w, int64_t M,
 }
 
 // ---------------------------------------------------------------------------
-// The right-looking panels of large launches: 64 items per CTA of 256 threads, in
-// shared memory (S[item][pos]).  The item threads eliminate tile T+1 while the
-// other warps still apply tile T's update (one barrier per tile), and the results
-// leave at the end, whole rows of the operand copies at a time.  Alone it takes as
-// long as the register variant with 64 items (27648 items 39 us); beside the bulk
-// update it is the faster one: whole factorizations on B200 with the register
-// variant / this, n = 8192 e4m3 4.11 / 3.83 ms, n = 16384 9.88 / 9.17, n = 24576
-// 23.0 / 21.7, n = 32768 46.8 / 44.2.
+// The panels of large right-looking launches beside tensor-core updates: 64 items
+// per CTA of 256 threads, in shared memory (S[item][pos]).  The item threads
+// eliminate tile T+1 while the other warps still apply tile T's update (one barrier
+// per tile), and the results leave at the end, whole rows of the operand copies at
+// a time.  Alone it takes as long as the register variant with 64 items (27648
+// items 39 us); beside the bulk update it is the faster one: whole factorizations
+// on B200 with the register variant / this, n = 8192 e4m3 4.11 / 3.85 ms, n = 16384
+// 9.88 / 9.2, n = 24576 23.0 / 21.7, n = 32768 46.8 / 44.2.
 constexpr int kWideThreads = 256;
 constexpr int kWideItems = 64;             // rows / columns per CTA
 constexpr int kMicroI = 4, kMicroP = 8;    // register micro-tile
@@ -1203,7 +1204,8 @@ lu_status launch_lupanel(cudaStream_t st, float* dg, int64_t lda, int w,
   const bool small = ceil_div(M, 32) + ceil_div(N, 32) <= sm_count();
   const auto fn = left    ? (small ? launch_lupanel_items<true, 32> : launch_lupanel_items<true, 64>)
                   : small ? launch_lupanel_items<false, 32>
-                          : launch_lupanel_wide;
+                  : pk.simt ? launch_lupanel_items<false, 64>
+                            : launch_lupanel_wide;
   return fn(st, dg, lda, w, M, N, offL, offU, pk);
 }
 
